@@ -240,14 +240,24 @@ inline int plan_problem(const fcr_problem& p, int num_sms, fcr_plan& pl, std::st
   }
   pl.row_items = (int32_t)row_items;
   pl.col_items = (int32_t)col_items;
-  // With the causal mask the items of a head shrink towards its end: interleave the
-  // heads whose Q and K (fp16) total at most 128 MiB (32 heads at most; measured flat from 16 to 32),
-  // so that the tail of the grid is made of the lightest items of many heads.  Without
-  // the mask all items weigh the same and one head at a time keeps the CTAs in step.
+  // With the causal mask the items of a head shrink towards its end: interleave heads, so that the tail
+  // of the grid is made of the lightest items of many heads.  All heads when their Q and K total at most
+  // 128 MiB (the L2 cache); else equal groups of at most 32 heads and 128 MiB (measured flat from 16 to
+  // 32 heads) -- equal, because a small last group would start its heaviest items when the others have
+  // finished (40 heads of 3001^2, d = 80: groups of 32 + 8 took 155 us, all 40 together take 136; 64 heads
+  // of 2048^2 in fp32: 32 + 32 took 115.6 us, all 64 take 109.5).  Without the mask all items weigh the same
+  // and one head at a time keeps the CTAs in step.
   const int64_t head_bytes = ((int64_t)p.M + p.N) * pl.d_pad * 2;
-  pl.head_group = !causal ? 1
-                          : (int32_t)std::max<int64_t>(
-                                1, std::min<int64_t>(std::min<int64_t>(BH, 32), (128LL << 20) / head_bytes));
+  int64_t group = 1;
+  if (causal) {
+    const int64_t fit = std::max<int64_t>(1, std::min<int64_t>(BH, (128LL << 20) / head_bytes));
+    group = fit;
+    if (fit < BH) {
+      group = std::min<int64_t>(fit, 32);
+      group = ceil_div64(BH, ceil_div64(BH, group));
+    }
+  }
+  pl.head_group = (int32_t)group;
   // Items that stream at most 8 tiles get the double-buffered stationary stage.
   pl.short_items = (ceil_div64(row_len, pl.row_splits) <= 8 ? 1 : 0) |
                    (ceil_div64(col_len, pl.col_splits) <= 8 ? 2 : 0);
