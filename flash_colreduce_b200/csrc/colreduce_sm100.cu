@@ -295,7 +295,7 @@ pass_kernel(const __grid_constant__ CUtensorMap tmap_stat,
     return g;
   };
 
-  const int warp = (int)(threadIdx.x >> 5);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // warp-uniform for the compiler
   const int lane = (int)(threadIdx.x & 31);
 
   if (warp == 0) {  // the lanes of one warp initialise the barriers side by side
@@ -524,24 +524,23 @@ pass_kernel(const __grid_constant__ CUtensorMap tmap_stat,
               if (!ok) break;
             }
             ptx::tc_fence_after_sync();
-            if (lane == 0) {
+            if (ptx::elect_one()) {
               const uint32_t d = tmem_base + (uint32_t)(a * 2 + ts) * kTile;
               const uint32_t b_addr = s_ring + s * L::kSlotBytes;
-              // One instruction per 32 bytes of each operand row: 16 halves or 8 TF32 values.
+              // One instruction per 32 bytes of each operand row: 16 halves or 8 TF32 values.  What a tile costs
+              // its issuer is the instructions around the MMAs, not the MMAs: with two 64-bit descriptors put
+              // together per step and a lane test that made every operand divergent, a tile of eight took 850
+              // cycles to issue (its MMAs take 512); with the descriptors' lower halves stepped by a constant
+              // under an elected lane 610.  8 heads of 131072^2: 38.7 -> 38.1 ms; 512 heads of 1024^2: 380 -> 371 us.
               // The operand kind is chosen once, outside the unrolled sequence.
               constexpr int kSteps = DPAD / 16 / L::kPieces;  // instructions per ring slot
+              const uint32_t a_lo = ptx::smem_desc_lo(a_addr) + piece * (L::kSlotHalves * (L::kHalfBytes >> 4));
+              const uint32_t b_lo = ptx::smem_desc_lo(b_addr);
               auto issue_steps = [&](auto as_tf32) {
 #pragma unroll
                 for (int kq = 0; kq < kSteps; ++kq) {
-                  const int kk = piece * kSteps + kq;  // step within the whole row
-                  const uint32_t a_off = (uint32_t)(kk >> 2) * L::kHalfBytes + (uint32_t)(kk & 3) * 32u;
-                  const uint32_t b_off = (uint32_t)(kq >> 2) * L::kHalfBytes + (uint32_t)(kq & 3) * 32u;
-                  if constexpr (decltype(as_tf32)::value)
-                    ptx::umma_tf32(d, ptx::smem_desc_sw128(a_addr + a_off),
-                                   ptx::smem_desc_sw128(b_addr + b_off), p.idesc, kk > 0 ? 1u : 0u);
-                  else
-                    ptx::umma_f16(d, ptx::smem_desc_sw128(a_addr + a_off),
-                                  ptx::smem_desc_sw128(b_addr + b_off), p.idesc, kk > 0 ? 1u : 0u);
+                  const uint32_t off = (uint32_t)(kq >> 2) * (L::kHalfBytes >> 4) + (uint32_t)(kq & 3) * 2u;
+                  ptx::umma_step<decltype(as_tf32)::value>(d, a_lo + off, b_lo + off, p.idesc, piece == 0 && kq == 0);
                 }
               };
               if (p.tf32)
@@ -563,7 +562,7 @@ pass_kernel(const __grid_constant__ CUtensorMap tmap_stat,
         }
       }
       if (!ok) break;
-      if (lane == 0) ptx::umma_commit(bar_stat_empty(ks));
+      if (ptx::elect_one()) ptx::umma_commit(bar_stat_empty(ks));
       __syncwarp();
     }
     if (ok && item_seq > 0) {

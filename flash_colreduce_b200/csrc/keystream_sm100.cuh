@@ -81,7 +81,7 @@ keystream_kernel(const __grid_constant__ CUtensorMap tmap_q,
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + L::off_misc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::off_misc + 4);
 
-  const int warp = (int)(threadIdx.x >> 5);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // warp-uniform for the compiler
   const int lane = (int)(threadIdx.x & 31);
 
   if (threadIdx.x == 0) {
@@ -186,22 +186,18 @@ keystream_kernel(const __grid_constant__ CUtensorMap tmap_q,
         if (!ok) break;
         tm_par ^= 1u << buf;
         ptx::tc_fence_after_sync();
-        if (lane == 0) {
+        if (ptx::elect_one()) {
           const uint32_t d = tmem_base + buf * kTile;
           const uint32_t k_addr = s_ring + s * L::kTileBytes;
           // rows pass: lanes = queries (A = query tile); columns pass: lanes = keys (A = key tile)
           const uint32_t a_addr = PHASE == PH_ROWS ? s_q : k_addr;
           const uint32_t b_addr = PHASE == PH_ROWS ? k_addr : s_q;
+          const uint32_t a_lo = ptx::smem_desc_lo(a_addr), b_lo = ptx::smem_desc_lo(b_addr);
           auto issue_steps = [&](auto as_tf32) {
 #pragma unroll
             for (int kk = 0; kk < DPAD / 16; ++kk) {
-              const uint32_t koff = (uint32_t)(kk >> 2) * L::kHalfBytes + (uint32_t)(kk & 3) * 32u;
-              if constexpr (decltype(as_tf32)::value)
-                ptx::umma_tf32(d, ptx::smem_desc_sw128(a_addr + koff),
-                               ptx::smem_desc_sw128(b_addr + koff), p.idesc, kk > 0 ? 1u : 0u);
-              else
-                ptx::umma_f16(d, ptx::smem_desc_sw128(a_addr + koff),
-                              ptx::smem_desc_sw128(b_addr + koff), p.idesc, kk > 0 ? 1u : 0u);
+              const uint32_t koff = (uint32_t)(kk >> 2) * (L::kHalfBytes >> 4) + (uint32_t)(kk & 3) * 2u;
+              ptx::umma_step<decltype(as_tf32)::value>(d, a_lo + koff, b_lo + koff, p.idesc, kk == 0);
             }
           };
           if (p.tf32)
@@ -217,7 +213,7 @@ keystream_kernel(const __grid_constant__ CUtensorMap tmap_q,
       // last item of this head on this CTA: the query tile may be replaced once these MMAs retire
       const int next_bh = (item + 1 < item_hi) ? (item + 1) / S : -1;
       if (next_bh != bh) {
-        if (lane == 0) ptx::umma_commit(bar_q_empty);
+        if (ptx::elect_one()) ptx::umma_commit(bar_q_empty);
         __syncwarp();
       }
     }

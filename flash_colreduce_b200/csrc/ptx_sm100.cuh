@@ -107,29 +107,68 @@ __device__ __forceinline__ void tc_fence_before_sync() {
 __device__ __forceinline__ void tc_fence_after_sync() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// D[tmem] (+)= A[smem] * B[smem]^T, fp16/bf16 operands, fp32 accumulate, one CTA.
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                         uint32_t idesc, uint32_t accumulate) {
+// Shared-memory matrix descriptor for a K-major operand tile stored as rows of 128 bytes with the
+// 128-byte swizzle (what a TMA box of 64 fp16 x rows with CU_TENSOR_MAP_SWIZZLE_128B writes): 8-row
+// groups are 1024 bytes apart.  The upper half is the same for every operand; the lower half holds the
+// start address in 16-byte units, so that a step along the row is one 32-bit addition (no carry:
+// shared memory ends below 2^18).
+constexpr uint32_t kDescHi = (1024u >> 4)   // stride byte offset: 8 rows * 128 B
+                             | (1u << 14)   // descriptor version (sm_100)
+                             | (2u << 29);  // layout: 128-byte swizzle
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t smem_addr) {
+  return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16);  // leading byte offset (unused here)
+}
+// One lane of a fully active warp, the same one every time; the code under it stays warp-uniform for
+// the compiler, which matters for tcgen05.mma: its operands live in uniform registers.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t on;
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
       "}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "=r"(on));
+  return on != 0;
+}
+// D[tmem] (+)= A[smem] * B[smem]^T, fp16/bf16 operands, fp32 accumulate, one CTA.
+template <bool ACCUMULATE>
+__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %4};\n\t"
+      "mov.b64 db, {%2, %4};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t"
+      "}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kDescHi), "n"(ACCUMULATE ? 1 : 0)
       : "memory");
 }
 // Same for fp32 operands taken as TF32 (K = 8 per instruction: again 32 bytes of each row).
-__device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                          uint32_t idesc, uint32_t accumulate) {
+template <bool ACCUMULATE>
+__device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc) {
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t"
+      ".reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %4};\n\t"
+      "mov.b64 db, {%2, %4};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %3, p;\n\t"
       "}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kDescHi), "n"(ACCUMULATE ? 1 : 0)
       : "memory");
+}
+// Step `kk` (32 bytes of each operand row) of a tile product; the first step overwrites D.
+template <bool TF32>
+__device__ __forceinline__ void umma_step(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, bool first) {
+  if (first) {
+    if constexpr (TF32) umma_tf32<false>(d_tmem, a_lo, b_lo, idesc); else umma_f16<false>(d_tmem, a_lo, b_lo, idesc);
+  } else {
+    if constexpr (TF32) umma_tf32<true>(d_tmem, a_lo, b_lo, idesc); else umma_f16<true>(d_tmem, a_lo, b_lo, idesc);
+  }
 }
 // Arrive on `bar` once every tcgen05 operation issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
@@ -228,20 +267,6 @@ __device__ __forceinline__ float2 ex2_poly2(float2 x) {
   r.x = __int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23));
   r.y = __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23));
   return r;
-}
-
-// ------------------------------------------------- tcgen05 descriptor helpers
-// Shared-memory matrix descriptor for a K-major operand tile stored as rows of
-// 128 bytes with the 128-byte swizzle (what a TMA box of 64 fp16 x rows with
-// CU_TENSOR_MAP_SWIZZLE_128B writes): 8-row groups are 1024 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);  // start address, 16-byte units
-  d |= static_cast<uint64_t>(1) << 16;                      // leading byte offset (unused here)
-  d |= static_cast<uint64_t>(1024 >> 4) << 32;              // stride byte offset: 8 rows * 128 B
-  d |= static_cast<uint64_t>(1) << 46;                      // descriptor version (sm_100)
-  d |= static_cast<uint64_t>(2) << 61;                      // layout: 128-byte swizzle
-  return d;
 }
 
 }  // namespace ptx
