@@ -105,6 +105,7 @@ struct PassParams : PassGeom {
   uint32_t idesc;  // tcgen05 instruction descriptor
   int tf32;        // fp32 operands multiplied as TF32 (else fp16 / bf16)
   int slab_elems;  // elements per 128-byte operand slab: 64 (16-bit) or 32 (fp32)
+  int k_steps;     // 32-byte steps of an operand row that hold data: the MMAs of a tile (rows are padded to 128 / 256 / 512 bytes)
   float* neg_lse;  // [BH][m_pad]
   float* part_m;   // [n_split][BH][m_pad]
   float* part_l;   // [n_split][BH][m_pad]
@@ -536,11 +537,21 @@ pass_kernel(const __grid_constant__ CUtensorMap tmap_stat,
               constexpr int kSteps = DPAD / 16 / L::kPieces;  // instructions per ring slot
               const uint32_t a_lo = ptx::smem_desc_lo(a_addr) + piece * (L::kSlotHalves * (L::kHalfBytes >> 4));
               const uint32_t b_lo = ptx::smem_desc_lo(b_addr);
+              auto issue_step = [&](auto as_tf32, int kq) {
+                const uint32_t off = (uint32_t)(kq >> 2) * (L::kHalfBytes >> 4) + (uint32_t)(kq & 3) * 2u;
+                ptx::umma_step<decltype(as_tf32)::value>(d, a_lo + off, b_lo + off, p.idesc, piece == 0 && kq == 0);
+              };
               auto issue_steps = [&](auto as_tf32) {
+                // Steps of this slot that hold data: a row is padded with zeros to 128, 256 or 512 bytes, and
+                // multiplying the padding is work for nothing (40 heads of 3001^2 with d = 80, 5 of 8 steps:
+                // 134 -> 128 us).  Full rows keep the unrolled sequence.
+                const int here = p.k_steps - piece * kSteps;
+                if (here >= kSteps) {
 #pragma unroll
-                for (int kq = 0; kq < kSteps; ++kq) {
-                  const uint32_t off = (uint32_t)(kq >> 2) * (L::kHalfBytes >> 4) + (uint32_t)(kq & 3) * 2u;
-                  ptx::umma_step<decltype(as_tf32)::value>(d, a_lo + off, b_lo + off, p.idesc, piece == 0 && kq == 0);
+                  for (int kq = 0; kq < kSteps; ++kq) issue_step(as_tf32, kq);
+                } else {
+#pragma unroll 1
+                  for (int kq = 0; kq < here; ++kq) issue_step(as_tf32, kq);
                 }
               };
               if (p.tf32)
@@ -1142,6 +1153,7 @@ static void fill_common(PassParams& pp, const fcr_problem& pr, const fcr_plan& p
   pp.idesc = instr_desc(pr.in_dtype, pr.scale < 0.f);
   pp.tf32 = pr.in_dtype == FCR_F32 ? 1 : 0;
   pp.slab_elems = pr.in_dtype == FCR_F32 ? 32 : 64;
+  pp.k_steps = (pr.D * (pr.in_dtype == FCR_F32 ? 4 : 2) + 31) / 32;
   pp.neg_lse = reinterpret_cast<float*>(ws + pl.off_neg_lse);
   pp.part_m = reinterpret_cast<float*>(ws + pl.off_part_m);
   pp.part_l = reinterpret_cast<float*>(ws + pl.off_part_l);
