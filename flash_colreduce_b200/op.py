@@ -7,6 +7,7 @@ Triton path and no CPU or eager fallback.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import math
 import os
@@ -46,6 +47,10 @@ def _tma_ready(x: torch.Tensor) -> torch.Tensor:
     return x if ok else x.contiguous()
 
 
+# What a call signature (shapes, strides, types, devices, options; no data, no addresses) comes to: whether each
+# operand can be described to TMA as it lies, the problem struct and the workspace size.  Small calls are bound by
+# the host, so a repeated signature is checked and planned once.
+_CALL_CACHE: dict = {}
 _PLAN_CACHE: dict = {}
 
 
@@ -63,6 +68,42 @@ def _problem_and_workspace_bytes(key_tuple, device):
     return hit
 
 
+def _on_device(index):
+    """Context that makes device ``index`` current: nothing at all when it already is."""
+    return _NO_CONTEXT if torch.cuda.current_device() == index else torch.cuda.device(index)
+
+
+_NO_CONTEXT = contextlib.nullcontext()
+
+
+def _queue(prob, ws_bytes, q, k, out, out_code):
+    """Allocates the workspace and queues the kernels on the current stream."""
+    index = q.device.index
+    with _on_device(index):
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
+        stream = torch._C._cuda_getCurrentRawStream(index)
+        rc = nat.lib.fcr_colreduce(C.byref(prob), q.data_ptr(), k.data_ptr(), out.data_ptr(), out_code,
+                                   ws.data_ptr(), ws_bytes, stream)
+        if rc:
+            nat.check(rc, "fcr_colreduce")
+        if _debug_sync():
+            nat.check(nat.lib.fcr_read_device_status(ws.data_ptr(), stream, None), "fcr_colreduce (device)")
+    return out
+
+
+def _prepare(query, key, reduction_code, is_causal, scale, causal_offset, mean_M, mean_N):
+    """The operands as TMA can describe them, the problem struct and the workspace size (cached)."""
+    b, h, m, _ = query.shape
+    n = key.shape[2]
+    q = _tma_ready(query)
+    k = _tma_ready(key)
+    d = q.shape[-1]
+    prob, ws_bytes = _problem_and_workspace_bytes(
+        (b, h, m, n, d, tuple(q.stride()), tuple(k.stride()), _DTYPE_CODES[q.dtype], reduction_code, bool(is_causal),
+         float(scale), int(causal_offset), int(mean_M), int(mean_N), q.device.index), q.device)
+    return q, k, prob, ws_bytes
+
+
 def _launch(query, key, out, out_code, reduction_code, is_causal, scale, causal_offset, mean_M, mean_N):
     """Plans (cached), allocates the workspace and queues the kernels on the current stream.
 
@@ -72,23 +113,8 @@ def _launch(query, key, out, out_code, reduction_code, is_causal, scale, causal_
     ``RuntimeError``.  ``FCR_DEBUG_SYNC=1`` additionally synchronises after every call and reads
     the status words of the call's own workspace.
     """
-    b, h, m, _ = query.shape
-    n = key.shape[2]
-    q = _tma_ready(query)
-    k = _tma_ready(key)
-    d = q.shape[-1]
-    prob, ws_bytes = _problem_and_workspace_bytes(
-        (b, h, m, n, d, tuple(q.stride()), tuple(k.stride()), _DTYPE_CODES[q.dtype], reduction_code, bool(is_causal),
-         float(scale), int(causal_offset), int(mean_M), int(mean_N), q.device.index), q.device)
-    with torch.cuda.device(q.device):
-        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-        stream = torch.cuda.current_stream(q.device).cuda_stream
-        rc = nat.lib.fcr_colreduce(C.byref(prob), q.data_ptr(), k.data_ptr(), out.data_ptr(), out_code,
-                                   ws.data_ptr(), ws.numel(), stream)
-        nat.check(rc, "fcr_colreduce")
-        if _debug_sync():
-            nat.check(nat.lib.fcr_read_device_status(ws.data_ptr(), stream, None), "fcr_colreduce (device)")
-    return out
+    q, k, prob, ws_bytes = _prepare(query, key, reduction_code, is_causal, scale, causal_offset, mean_M, mean_N)
+    return _queue(prob, ws_bytes, q, k, out, out_code)
 
 
 def _validate(query: torch.Tensor, key: torch.Tensor, reduction: str) -> None:
@@ -142,6 +168,16 @@ def flash_colreduce(
         (B, H, N) tensor of ``query.dtype``.  Accumulation is fp32 and the
         result is rounded once; run-to-run results are bitwise identical.
     """
+    is_causal = bool(is_causal)
+    if scale is not None:
+        scale = float(scale)
+    signature = (query.shape, key.shape, query.stride(), key.stride(), query.dtype, key.dtype, query.device,
+                 key.device, reduction, is_causal, scale)
+    hit = _CALL_CACHE.get(signature) if type(reduction) is str else None
+    if hit is not None and query.data_ptr() % 16 == 0 and key.data_ptr() % 16 == 0:
+        prob, ws_bytes, out_shape, out_code = hit
+        out = torch.empty(out_shape, dtype=query.dtype, device=query.device)
+        return _queue(prob, ws_bytes, query, key, out, out_code)
     _validate(query, key, reduction)
     b, h, m, d = query.shape
     n = key.shape[2]
@@ -154,8 +190,13 @@ def flash_colreduce(
         # no query contributes: zeros for sum / max, 0/0 for mean as in the reference
         out.zero_()
         return out / 0 if reduction == "mean" else out
-    return _launch(query, key, out, _DTYPE_CODES[out.dtype], nat.REDUCTION_CODES[reduction], is_causal,
-                   scale, -1, 0, 0)
+    out_code = _DTYPE_CODES[out.dtype]
+    q, k, prob, ws_bytes = _prepare(query, key, nat.REDUCTION_CODES[reduction], is_causal, scale, -1, 0, 0)
+    if q is query and k is key:  # both operands go in as they lie
+        if len(_CALL_CACHE) > 4096:
+            _CALL_CACHE.clear()
+        _CALL_CACHE[signature] = (prob, ws_bytes, (b, h, n), out_code)
+    return _queue(prob, ws_bytes, q, k, out, out_code)
 
 
 def colreduce_partial(
@@ -216,17 +257,20 @@ def topk_columns(scores: torch.Tensor, k: int, return_values: bool = True):
     n = scores.shape[-1]
     if not 1 <= k <= n:
         raise ValueError(f"k = {k} must lie in [1, {n}].")
-    flat = scores.contiguous().view(-1, n)
-    lead = scores.shape[:-1]
-    indices = torch.empty((flat.shape[0], k), dtype=torch.int64, device=scores.device)
-    values = torch.empty((flat.shape[0], k), dtype=scores.dtype, device=scores.device) if return_values else None
-    if flat.shape[0] > 0:
-        with torch.cuda.device(scores.device):
-            stream = torch.cuda.current_stream(scores.device).cuda_stream
-            rc = nat.lib.fcr_topk(flat.data_ptr(), _DTYPE_CODES[scores.dtype], flat.shape[0], n, k,
-                                  indices.data_ptr(), 64, values.data_ptr() if return_values else None, stream)
-            nat.check(rc, "fcr_topk")
-    return (values.view(*lead, k) if return_values else None), indices.view(*lead, k)
+    flat = scores if scores.is_contiguous() else scores.contiguous()
+    shape = (*scores.shape[:-1], k)
+    rows = flat.numel() // n
+    indices = torch.empty(shape, dtype=torch.int64, device=scores.device)
+    values = torch.empty(shape, dtype=scores.dtype, device=scores.device) if return_values else None
+    if rows > 0:
+        index = scores.device.index
+        with _on_device(index):
+            rc = nat.lib.fcr_topk(flat.data_ptr(), _DTYPE_CODES[scores.dtype], rows, n, k, indices.data_ptr(), 64,
+                                  values.data_ptr() if return_values else None,
+                                  torch._C._cuda_getCurrentRawStream(index))
+            if rc:
+                nat.check(rc, "fcr_topk")
+    return values, indices
 
 
 def select_columns(scores: torch.Tensor, threshold: float):
