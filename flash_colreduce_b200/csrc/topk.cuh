@@ -56,6 +56,18 @@ struct TopkKey<__nv_bfloat16> {
   }
 };
 
+// The score a key was made from (the map is one to one: the score's own bits come back).
+__device__ __forceinline__ void topk_score(uint32_t key, float& x) {
+  x = __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
+}
+__device__ __forceinline__ unsigned short topk_score_bits16(uint32_t key) {
+  return (unsigned short)((key & 0x8000u) ? (key & 0x7fffu) : ~key);
+}
+__device__ __forceinline__ void topk_score(uint32_t key, __half& x) { x = __ushort_as_half(topk_score_bits16(key)); }
+__device__ __forceinline__ void topk_score(uint32_t key, __nv_bfloat16& x) {
+  x = __ushort_as_bfloat16(topk_score_bits16(key));
+}
+
 // Keys of elements [i0, i0 + 8) of a row (unspecified beyond n); 16-byte loads when the address allows.
 template <typename T>
 __device__ __forceinline__ void topk_load8(const T* row, int i0, int n, uint32_t (&key)[kTopkItems]) {
@@ -104,6 +116,29 @@ topk_kernel(const T* __restrict__ scores, int n, int k, IndexT* __restrict__ ind
   const int lo = (int)(((long long)n * rank / n_ranks) & ~7LL);
   const int hi = rank + 1 == n_ranks ? n : (int)(((long long)n * (rank + 1) / n_ranks) & ~7LL);
 
+  // A slice of at most one sweep step stays in registers: it is read once for all rounds, and the values
+  // written are made from the keys.  Such a row is a chain of latencies (load, two or four histogram rounds,
+  // scan), not bandwidth: 128 rows of 8192 fp16 scores took 9.85 us with three reads of the row and cluster
+  // barriers in a cluster of one, 9.1 us with one read and block barriers.
+  const bool resident = hi - lo <= kStep;
+  uint32_t held[kTopkItems];
+  if (resident) topk_load8<T>(row, lo + tid * kTopkItems, hi, held);
+  auto load_keys = [&](int i0, uint32_t (&key)[kTopkItems]) {
+    if (resident) {
+#pragma unroll
+      for (int j = 0; j < kTopkItems; ++j) key[j] = held[j];
+    } else {
+      topk_load8<T>(row, i0, hi, key);
+    }
+  };
+  // a barrier over the CTAs of the row
+  auto sync_row = [&]() {
+    if (n_ranks > 1)
+      cluster.sync();
+    else
+      __syncthreads();
+  };
+
   // ---- radix select: after the last round `prefix` is the key of the k-th largest element
   uint32_t prefix = 0, mask = 0, want = (uint32_t)k;
   for (int shift = TopkKey<T>::kBits - 8; shift >= 0; shift -= 8) {
@@ -113,7 +148,7 @@ topk_kernel(const T* __restrict__ scores, int n, int k, IndexT* __restrict__ ind
     for (int c0 = lo; c0 < hi; c0 += kStep) {
       const int i0 = c0 + tid * kTopkItems;
       uint32_t key[kTopkItems];
-      topk_load8<T>(row, i0, hi, key);
+      load_keys(i0, key);
 #pragma unroll
       for (int j = 0; j < kTopkItems; ++j) {
         if (i0 + j < hi && (key[j] & mask) == prefix)
@@ -128,14 +163,14 @@ topk_kernel(const T* __restrict__ scores, int n, int k, IndexT* __restrict__ ind
       for (int j = 0; j < COPIES; ++j) total += hist[tid * COPIES + ((j + lane) & (COPIES - 1))];
       bin_total[tid] = total;
     }
-    cluster.sync();  // every slice's totals are complete (also a barrier of this CTA)
+    sync_row();  // every slice's totals are complete (also a barrier of this CTA)
     if (warp == 0) {
       // lane L owns bins [8L, 8L + 8), summed over the slices; `above` = elements in higher bins
       uint32_t bins[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) bins[j] = 0;
       for (int r = 0; r < n_ranks; ++r) {
-        const int* remote = cluster.map_shared_rank(bin_total, r);
+        const int* remote = n_ranks > 1 ? cluster.map_shared_rank(bin_total, r) : bin_total;
 #pragma unroll
         for (int j = 0; j < 8; ++j) bins[j] += (uint32_t)remote[lane * 8 + j];
       }
@@ -162,7 +197,7 @@ topk_kernel(const T* __restrict__ scores, int n, int k, IndexT* __restrict__ ind
         s_want = want - above;  // how many elements of that bin are still needed
       }
     }
-    cluster.sync();  // the totals have been read everywhere: they may be rebuilt in the next round
+    sync_row();  // the totals have been read everywhere: they may be rebuilt in the next round
     prefix = s_prefix;
     want = s_want;
     mask |= 255u << shift;
@@ -179,7 +214,7 @@ topk_kernel(const T* __restrict__ scores, int n, int k, IndexT* __restrict__ ind
     for (int c0 = lo; c0 < hi; c0 += kStep) {
       const int i0 = c0 + tid * kTopkItems;
       uint32_t key[kTopkItems];
-      topk_load8<T>(row, i0, hi, key);
+      load_keys(i0, key);
 #pragma unroll
       for (int j = 0; j < kTopkItems; ++j) {
         g += (i0 + j < hi && key[j] > thr) ? 1u : 0u;
@@ -204,7 +239,7 @@ topk_kernel(const T* __restrict__ scores, int n, int k, IndexT* __restrict__ ind
   for (int c0 = lo; c0 < hi; c0 += kStep) {
     const int i0 = c0 + tid * kTopkItems;
     uint32_t key[kTopkItems];
-    topk_load8<T>(row, i0, hi, key);
+    load_keys(i0, key);
     uint32_t g = 0, e = 0;
     bool isg[kTopkItems], ise[kTopkItems];
 #pragma unroll
@@ -244,7 +279,7 @@ topk_kernel(const T* __restrict__ scores, int n, int k, IndexT* __restrict__ ind
       if (isg[j] || (ise[j] && e_before < ties)) {
         const uint32_t pos = g_before + min(e_before, ties);
         out_idx[pos] = (IndexT)(i0 + j);
-        if (out_val) out_val[pos] = row[i0 + j];
+        if (out_val) topk_score(key[j], out_val[pos]);
       }
       g_before += isg[j];
       e_before += ise[j];
@@ -254,7 +289,7 @@ topk_kernel(const T* __restrict__ scores, int n, int k, IndexT* __restrict__ ind
     eq_base += tot >> 16;
     __syncthreads();  // warp_tot / chunk_tot are rewritten by the next step
   }
-  cluster.sync();  // no CTA leaves while another may still read its shared memory
+  sync_row();  // no CTA leaves while another may still read its shared memory
 }
 
 __device__ __forceinline__ float topk_to_float(float v) { return v; }
