@@ -759,6 +759,7 @@ pass_kernel(const __grid_constant__ CUtensorMap tmap_stat,
 
 }  // namespace fcr
 #include "keystream_sm100.cuh"
+#include "onesweep_sm100.cuh"
 #include "topk.cuh"
 namespace fcr {
 
@@ -917,10 +918,10 @@ static EncodeTiledFn encode_tiled_fn() {
 }
 
 // Tensor map over a (B,H,rows,D) tensor viewed as 4-D (D, rows, H, B); a box
-// is 64 elements x 128 rows of one head, written to shared memory with the
+// is 64 elements x 128 rows (or `box_rows`) of one head, written to shared memory with the
 // 128-byte swizzle.  Elements beyond D or beyond `rows` read as zero.
 static int make_tensor_map(CUtensorMap* map, const void* ptr, int dtype, int D, int rows, int H,
-                           int B, const int64_t* strides) {
+                           int B, const int64_t* strides, int box_rows = kTile) {
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return fail(FCR_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   if ((reinterpret_cast<uintptr_t>(ptr) & 15u) != 0)
@@ -935,7 +936,7 @@ static int make_tensor_map(CUtensorMap* map, const void* ptr, int dtype, int D, 
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)rows, (cuuint64_t)H, (cuuint64_t)B};
   cuuint64_t gstr[3] = {stride_bytes(rows, strides[2]), stride_bytes(H, strides[1]),
                         stride_bytes(B, strides[0])};
-  cuuint32_t box[4] = {(cuuint32_t)(128 / elem_bytes), (cuuint32_t)kTile, 1u, 1u};  // 128-byte slab
+  cuuint32_t box[4] = {(cuuint32_t)(128 / elem_bytes), (cuuint32_t)box_rows, 1u, 1u};  // 128-byte slab
   cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
   const CUtensorMapDataType dt = dtype == FCR_F32    ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                  : dtype == FCR_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
@@ -1124,20 +1125,51 @@ static int launch_keystream_d(int d_pad, const CUtensorMap& map_q, const CUtenso
   return launch_keystream<PHASE, 128, RED>(map_q, map_k, pp, ctas, stream);
 }
 
-// Bytes a plan cannot do without: the score cache is the last region of the workspace and is
-// optional (without it the columns pass sweeps K a second time).
-static int64_t min_workspace_bytes(const fcr_plan& pl) {
-  return pl.score_cache ? pl.off_scores : pl.workspace_bytes;
+// Returns the launch's own error: a grid that cannot be resident at once (a context with fewer SMs than
+// the device) is the caller's cue to run the two-sweep kernels instead.
+template <int DPAD, int RED>
+static cudaError_t launch_onesweep(const CUtensorMap& map_q, const CUtensorMap& map_k, const PassParams& pp,
+                                   float2* chunk_state, int* head_count, uint32_t idesc_cols, int copies, int ctas,
+                                   cudaStream_t stream) {
+  auto kern = onesweep_kernel<DPAD, RED>;
+  constexpr int smem = OneSweepSmem<DPAD>::kDynamicBytes;
+  static std::atomic<unsigned long long> opted_in{0};
+  cudaError_t e = cudaSuccess;
+  const unsigned long long bit = 1ULL << (t_device & 63);
+  if (!(opted_in.load(std::memory_order_acquire) & bit)) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    opted_in.fetch_or(bit, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(kOsThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, kern, map_q, map_k, pp, chunk_state, head_count, idesc_cols, copies);
+  if (e == cudaSuccess) g_launches.fetch_add(1, std::memory_order_relaxed);
+  return e;
 }
 
-static int check_workspace(const fcr_plan& pl, const void* ws, size_t ws_bytes) {
+// Bytes a plan cannot do without: the score cache and the one-sweep kernel's scratch are each the last
+// region of the workspace and optional (without them the columns pass sweeps K a second time).
+static int64_t min_workspace_bytes(const fcr_problem& pr, const fcr_plan& pl, int sms) {
+  return pl.score_cache ? pl.off_scores : pl.workspace_bytes - onesweep_bytes(pr, pl, sms);
+}
+
+static int check_workspace(const fcr_problem& pr, const fcr_plan& pl, int sms, const void* ws, size_t ws_bytes) {
+  const int64_t needed = min_workspace_bytes(pr, pl, sms);
   if (!ws) return fail(FCR_ERR_WORKSPACE, "workspace is null");
   if ((reinterpret_cast<uintptr_t>(ws) & 255u) != 0)
     return fail(FCR_ERR_WORKSPACE, "workspace must be 256-byte aligned");
-  if ((int64_t)ws_bytes < min_workspace_bytes(pl))
+  if ((int64_t)ws_bytes < needed)
     return fail(FCR_ERR_WORKSPACE, "workspace of " + std::to_string(ws_bytes) +
-                                       " bytes is smaller than the required " +
-                                       std::to_string(min_workspace_bytes(pl)));
+                                       " bytes is smaller than the required " + std::to_string(needed));
   return FCR_OK;
 }
 
@@ -1356,7 +1388,7 @@ static int plan_for_call(const fcr_problem& pr, const DeviceInfo& dev, const fcr
 static int run_colreduce(const fcr_problem& pr, const fcr_plan& pl, const DeviceInfo& dev, const void* q,
                          const void* k, void* out, int32_t out_dtype, void* workspace,
                          size_t workspace_bytes, cudaStream_t stream) {
-  int rc = check_workspace(pl, workspace, workspace_bytes);
+  int rc = check_workspace(pr, pl, dev.sms, workspace, workspace_bytes);
   if (rc != FCR_OK) return rc;
   uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
   t_device = dev.index;
@@ -1388,6 +1420,45 @@ static int run_colreduce(const fcr_problem& pr, const fcr_plan& pl, const Device
       pp.fold_cols = (int)align_up64(pr.M, kChunkCols);
     };
     fill(false);
+    // One sweep over K instead of two, when the workspace has room for the chunk states.
+    const int chunks = onesweep_chunks(pr, pl, dev.sms);
+    if (chunks > 0 && (int64_t)workspace_bytes >= pl.workspace_bytes) {
+      fill_mean(pp, pr.reduction, pr.is_causal, pr.mean_M > 0 ? pr.mean_M : pr.M,
+                pr.mean_N > 0 ? pr.mean_N : pr.N);
+      pp.out = out;
+      pp.out_dtype = out_dtype;
+      pp.n_split = chunks;
+      pp.n_items = pp.BH * chunks;
+      uint8_t* region = ws + (pl.workspace_bytes - onesweep_bytes(pr, pl, dev.sms));
+      int* head_count = reinterpret_cast<int*>(region);
+      float2* chunk_state = reinterpret_cast<float2*>(region + onesweep_counter_bytes(pr));
+      e = cudaMemsetAsync(head_count, 0, onesweep_counter_bytes(pr), stream);
+      if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(chunk counters)");
+      const int copies = onesweep_copies(pr.M);
+      CUtensorMap map_qc = map_q;
+      if (copies > 1) {
+        rc = make_tensor_map(&map_qc, q, pr.in_dtype, pr.D, pr.M, pr.H, pr.B, pr.q_strides, kTile / copies);
+        if (rc != FCR_OK) return rc;
+      }
+      // the columns segment multiplies against the query rows that exist, to the fold's granularity
+      const uint32_t idesc_cols = (pp.idesc & ~(63u << 17)) | ((uint32_t)(pp.fold_cols >> 3) << 17);
+      const int ctas = std::min(pp.n_items, dev.sms);
+      const bool is_max = pr.reduction == FCR_MAX;
+      if (pl.d_pad == 64)
+        e = is_max ? launch_onesweep<64, RED_MAX>(map_qc, map_k, pp, chunk_state, head_count, idesc_cols, copies, ctas, stream)
+                   : launch_onesweep<64, RED_SUM>(map_qc, map_k, pp, chunk_state, head_count, idesc_cols, copies, ctas, stream);
+      else
+        e = is_max ? launch_onesweep<128, RED_MAX>(map_qc, map_k, pp, chunk_state, head_count, idesc_cols, copies, ctas, stream)
+                   : launch_onesweep<128, RED_SUM>(map_qc, map_k, pp, chunk_state, head_count, idesc_cols, copies, ctas, stream);
+      if (e == cudaSuccess) {
+        trace_mark(1, stream);
+        trace_mark(2, stream);
+        return FCR_OK;
+      }
+      if (e != cudaErrorCooperativeLaunchTooLarge) return cuda_fail(e, "one-sweep kernel launch");
+      cudaGetLastError();  // clear it
+      fill(false);
+    }
     // the score cache is used when the caller's workspace has room for it
     const bool use_cache = pl.score_cache && (int64_t)workspace_bytes >= pl.workspace_bytes;
     if (use_cache) pp.dump = reinterpret_cast<float*>(ws + pl.off_scores);
@@ -1626,9 +1697,10 @@ int fcr_colreduce_static(const fcr_problem* problem, const void* q, const void* 
   const fcr_plan* pl = nullptr;
   rc = plan_for_call(*problem, *dev, &pl);
   if (rc != FCR_OK) return rc;
-  if ((size_t)min_workspace_bytes(*pl) > kStaticScratchBytes)
+  const int64_t needed = min_workspace_bytes(*problem, *pl, dev->sms);
+  if ((size_t)needed > kStaticScratchBytes)
     return fail(FCR_ERR_WORKSPACE,
-                "this problem needs " + std::to_string(min_workspace_bytes(*pl)) +
+                "this problem needs " + std::to_string(needed) +
                     " bytes of scratch but the built-in scratch holds " +
                     std::to_string(kStaticScratchBytes) +
                     " (FCR_STATIC_SCRATCH_BYTES); use fcr_colreduce with a caller-owned workspace");

@@ -161,6 +161,47 @@ inline int choose_splits(int64_t base_items, int64_t max_len_tiles, int num_sms)
   return best;
 }
 
+// One-sweep decode kernel (onesweep_sm100.cuh): chunks per head, 0 when the plan does not take it.
+// It takes the key-streaming shapes without a score cache whose operand rows span at most 256 bytes (two
+// query tiles of 64 KB would leave no room for a key ring).  CTA c runs chunks c, c + G, ... and reads a
+// chunk's tiles again one chunk later.  Unless all of K fits the L2 anyway, a chunk is at most 256 KB of K:
+// 16 x 32 heads, 64 x 16384, d = 128 took 1046 us with chunks of 3 tiles of 32 KB, 767 with 5, 665 with 8 and
+// 696 with 10 (two sweeps: 876), the small ones for the set-up of a chunk (about two tiles' time, the 2 in the
+// cost below), the large ones because the chunk has left the L2 before its second sweep.  S <= num_sms keeps
+// the waits between CTAs free of cycles.
+// With rows of 128 bytes and more than 64 queries the folds bind, not the reading of K, and the second sweep
+// saves nothing: 256 heads, 128 x 8192, d = 64 took 158 us in two sweeps, 167 in one.  Only where K fits the
+// L2, whose problems are bound by the launches and the combination instead (4 heads, 128 x 65536: 56 -> 32 us).
+constexpr int64_t kOneSweepL2Bytes = 40LL << 20;
+constexpr int64_t kOneSweepChunkBytes = 256 << 10;
+inline int onesweep_chunks(const fcr_problem& p, const fcr_plan& pl, int num_sms) {
+  if (!pl.key_stream || pl.score_cache || pl.d_pad > 128) return 0;
+  const int64_t BH = (int64_t)p.B * p.H, key_tiles = pl.n_pad / kTile, tile_bytes = (int64_t)kTile * pl.d_pad * 2;
+  const bool in_l2 = BH * key_tiles * tile_bytes <= kOneSweepL2Bytes;
+  if (!in_l2 && pl.d_pad == 64 && p.M > 64) return 0;
+  int best = 0;
+  int64_t best_cost = -1;
+  for (int64_t s = 1; s <= std::min<int64_t>(key_tiles, num_sms); ++s) {
+    const int64_t tiles = ceil_div64(key_tiles, s);
+    if (!in_l2 && tiles * tile_bytes > kOneSweepChunkBytes) continue;
+    const int64_t cost = ceil_div64(BH * s, num_sms) * (tiles + 2);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = (int)s;
+    }
+  }
+  return BH * best > (1LL << 30) ? 0 : best;
+}
+// Copies of the query tile stacked in the 128 rows of an MMA: the spare rows repeat the queries, so that
+// the warps of the spare lanes fold their own share of a key tile's columns.
+inline int onesweep_copies(int M) { return M <= 32 ? 4 : (M <= 64 ? 2 : 1); }
+// Its scratch, the last region of the workspace: int[B*H][4] chunk counters, float2[S][B*H][m_pad] chunk states.
+inline int64_t onesweep_counter_bytes(const fcr_problem& p) { return align_up64((int64_t)p.B * p.H * 4 * 4, 256); }
+inline int64_t onesweep_bytes(const fcr_problem& p, const fcr_plan& pl, int num_sms) {
+  const int64_t s = onesweep_chunks(p, pl, num_sms);
+  return s == 0 ? 0 : onesweep_counter_bytes(p) + align_up64(s * p.B * p.H * pl.m_pad * 8, 256);
+}
+
 inline int plan_problem(const fcr_problem& p, int num_sms, fcr_plan& pl, std::string& err) {
   pl = fcr_plan{};
   if (p.B <= 0 || p.H <= 0 || p.M <= 0 || p.N <= 0 || p.D <= 0) {
@@ -334,6 +375,7 @@ inline int plan_problem(const fcr_problem& p, int num_sms, fcr_plan& pl, std::st
     pl.off_scores = o;
     o += align_up64(score_bytes, 256);
   }
+  o += onesweep_bytes(p, pl, num_sms);
   pl.workspace_bytes = o;
   return FCR_OK;
 }

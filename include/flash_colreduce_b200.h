@@ -111,6 +111,10 @@ typedef struct fcr_plan {
                              * workspace and optional: a workspace of only off_scores bytes is accepted, the
                              * columns pass then sweeps K a second time */
   int32_t score_cache;      /* 1 when the columns are reduced from cached scores */
+  /* Key streaming without a score cache and with operand rows of at most 256 bytes: one kernel runs both
+   * passes chunk by chunk, so that K is read from HBM once, when the workspace has workspace_bytes bytes.
+   * Its scratch (chunk counters and chunk states) is the last region of the workspace and optional: a
+   * workspace that ends after off_part_l's array is accepted, and the two kernels described above run. */
   int32_t static_schedule;  /* 1: work items are dealt round-robin (item, item + CTAs, ...) and nothing in the workspace has
                              * to be cleared before the kernels (small problems and the key-streaming kernels);
                              * 0: CTAs draw items from a counter, which one cudaMemsetAsync per call clears */
@@ -201,7 +205,8 @@ int fcr_colreduce(const fcr_problem* problem, const void* q, const void* k, void
  *   shapes with a score cache (fcr_plan.score_cache): the cache is optional
  *   here as it is for fcr_colreduce, so for those the limit applies to
  *   fcr_plan.off_scores, and the cache is used when all of
- *   fcr_plan.workspace_bytes fits the array.
+ *   fcr_plan.workspace_bytes fits the array.  The scratch of the one-sweep decode
+ *   kernel is optional in the same way.
  * - The first call on each device looks up the array's device address (with
  *   that device current) and caches it; make that first call before any
  *   stream capture begins.
@@ -333,6 +338,7 @@ int fcr_self_test_hooks(int64_t wait_limit_cycles, int32_t skip_ring_load);
  * enabling resets the count).  fcr_trace_read synchronises on call `index`
  * and returns the device time of its rows pass (plus the split combine, if
  * any) and of its columns pass (plus the final reduction, if any).
+ * A call that one kernel runs (the one-sweep decode kernel) has all its time in rows_ms.
  */
 int fcr_trace_enable(int32_t on);
 int32_t fcr_trace_count(void);
