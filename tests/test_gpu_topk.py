@@ -141,3 +141,15 @@ def test_many_short_rows_inside_a_cuda_graph(monkeypatch):
     assert torch.equal(vals.cpu().float().sort(dim=-1, descending=True)[0], want_vals)
     fresh = flash_colreduce(q, key, "sum")
     assert torch.equal(fresh.cpu(), scores_cpu)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,n,k", [(3, 8191, 100), (3, 8192, 8192), (3, 8193, 2049), (2, 16384, 5000), (2, 16390, 5000),
+                                      (400, 2047, 300), (400, 2048, 1), (400, 2049, 2049)])
+def test_rows_at_the_edge_of_one_sweep_step(dtype, rows, n, k):
+    """A slice of one sweep step (8192 elements, 2048 for the small blocks) is kept in registers, one more element is
+    not; the values are made from the keys, so negative scores, both zeros and infinities come back bit for bit."""
+    g = torch.Generator().manual_seed(n + k)
+    s = torch.randn(rows, n, generator=g).to(dtype)
+    s[0, : min(4, n)] = torch.tensor([float("inf"), float("-inf"), 0.5, -0.5][: min(4, n)]).to(dtype)
+    _check(s, k)
