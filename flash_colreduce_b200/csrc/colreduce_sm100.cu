@@ -195,7 +195,9 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
     if (ptx::mbar_try_wait(bar, parity)) return true;
     if ((++spins & 7u) == 0) {
       if (*abort_flag) return false;
-      if (clock64() - t0 > p.wait_limit) {
+      // The TMA warp waits for slots that its consumers give back, so a consumer that is stuck makes it wait
+      // too, a few hundred cycles later: twice the bound for it, and the status names the wait at the root.
+      if (clock64() - t0 > (code < ST_WAIT_STAT_FULL ? 2 : 1) * p.wait_limit) {
         *abort_flag = 1;
         report_status(p, code, (int)parity);
         return false;
