@@ -1,4 +1,6 @@
-// Key-streaming kernels for the decode shapes: all M <= 128 queries of a head
+// Key-streaming kernels for the decode shapes, one per pass.  (For 16 < M <= 128 and rows of at
+// most 256 bytes onesweep_sm100.cuh runs both passes in one kernel, when the workspace has room;
+// these run M <= 16 with the score cache and whatever that one does not take.)  All M <= 128 queries of a head
 // fit one tile, the keys are long.  Both passes keep the query tile of the
 // current head in shared memory and stream that head's key tiles through a deep
 // ring whose slots are released as soon as the MMAs that read them have retired,
