@@ -338,6 +338,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             }
           }
         }
+        __syncwarp();  // lane 0's acquire covers the loads of all lanes (a vote orders no memory)
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         float mx = -INFINITY, l = 0.f;

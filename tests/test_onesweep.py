@@ -2,6 +2,7 @@
 import ctypes as C
 import math
 import os
+import re
 import subprocess
 
 import pytest
@@ -105,6 +106,17 @@ def test_schedule_covers_the_keys_and_never_waits_in_a_circle(planner, b, h, m, 
                 fold[c] += 1
                 moved = True
     assert all(fold[c] == 2 * (chunks[c] + lag) and len(fetched[c]) == chunks[c] for c in range(G)), "a CTA waits for good"
+
+
+def test_the_exchange_orders_the_memory_of_all_lanes():
+    """One lane of a statistics warp releases and acquires a head's counter for the loads and stores of all 32: a warp
+    barrier stands between the stores of a chunk state and the release, and between the acquire and the loads."""
+    with open(os.path.join(ROOT, "flash_colreduce_b200", "csrc", "onesweep_sm100.cuh")) as f:
+        code = re.sub(r"//[^\n]*", "", f.read())
+    assert code.count("red_release_add(") == 1 and code.count("__stcg(") == 1 and code.count("__ldcg(") == 1
+    publish = code[code.index("__stcg("):code.index("red_release_add(")]
+    collect = code[code.rindex("ld_acquire("):code.index("__ldcg(")]
+    assert "__syncwarp()" in publish and "__syncwarp()" in collect
 
 
 def test_which_shapes_take_it_and_where_its_scratch_lies(planner):
