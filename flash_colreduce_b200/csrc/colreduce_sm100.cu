@@ -1127,12 +1127,10 @@ static int launch_keystream_d(int d_pad, const CUtensorMap& map_q, const CUtenso
   return launch_keystream<PHASE, 128, RED>(map_q, map_k, pp, ctas, stream);
 }
 
-// Returns the launch's own error: a grid that cannot be resident at once (a context with fewer SMs than
-// the device) is the caller's cue to run the two-sweep kernels instead.
 template <int DPAD, int RED>
-static cudaError_t launch_onesweep(const CUtensorMap& map_q, const CUtensorMap& map_k, const PassParams& pp,
-                                   float2* chunk_state, int* head_count, uint32_t idesc_cols, int copies, int ctas,
-                                   cudaStream_t stream) {
+static int launch_onesweep(const CUtensorMap& map_q, const CUtensorMap& map_k, const PassParams& pp,
+                           float2* chunk_state, int* counters, uint32_t idesc_cols, int copies, int ctas,
+                           cudaStream_t stream) {
   auto kern = onesweep_kernel<DPAD, RED>;
   constexpr int smem = OneSweepSmem<DPAD>::kDynamicBytes;
   static std::atomic<unsigned long long> opted_in{0};
@@ -1140,22 +1138,23 @@ static cudaError_t launch_onesweep(const CUtensorMap& map_q, const CUtensorMap& 
   const unsigned long long bit = 1ULL << (t_device & 63);
   if (!(opted_in.load(std::memory_order_acquire) & bit)) {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
     opted_in.fetch_or(bit, std::memory_order_release);
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(kOsThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, kern, map_q, map_k, pp, chunk_state, head_count, idesc_cols, copies);
-  if (e == cudaSuccess) g_launches.fetch_add(1, std::memory_order_relaxed);
-  return e;
+  e = launch_kernel(kern, dim3(ctas), dim3(kOsThreads), smem, stream, false, map_q, map_k, pp, chunk_state, counters,
+                    counters + (size_t)pp.BH * kOsStatWarps, idesc_cols, copies);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(e, "one-sweep kernel launch");
+  return FCR_OK;
+}
+
+template <int RED>
+static int launch_onesweep_d(int d_pad, const CUtensorMap& map_q, const CUtensorMap& map_k, const PassParams& pp,
+                             float2* chunk_state, int* counters, uint32_t idesc_cols, int copies, int ctas,
+                             cudaStream_t stream) {
+  if (d_pad == 64)
+    return launch_onesweep<64, RED>(map_q, map_k, pp, chunk_state, counters, idesc_cols, copies, ctas, stream);
+  return launch_onesweep<128, RED>(map_q, map_k, pp, chunk_state, counters, idesc_cols, copies, ctas, stream);
 }
 
 // Bytes a plan cannot do without: the score cache and the one-sweep kernel's scratch are each the last
@@ -1432,9 +1431,9 @@ static int run_colreduce(const fcr_problem& pr, const fcr_plan& pl, const Device
       pp.n_split = chunks;
       pp.n_items = pp.BH * chunks;
       uint8_t* region = ws + (pl.workspace_bytes - onesweep_bytes(pr, pl, dev.sms));
-      int* head_count = reinterpret_cast<int*>(region);
+      int* counters = reinterpret_cast<int*>(region);
       float2* chunk_state = reinterpret_cast<float2*>(region + onesweep_counter_bytes(pr));
-      e = cudaMemsetAsync(head_count, 0, onesweep_counter_bytes(pr), stream);
+      e = cudaMemsetAsync(counters, 0, onesweep_counter_bytes(pr), stream);
       if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(chunk counters)");
       const int copies = onesweep_copies(pr.M);
       CUtensorMap map_qc = map_q;
@@ -1445,21 +1444,13 @@ static int run_colreduce(const fcr_problem& pr, const fcr_plan& pl, const Device
       // the columns segment multiplies against the query rows that exist, to the fold's granularity
       const uint32_t idesc_cols = (pp.idesc & ~(63u << 17)) | ((uint32_t)(pp.fold_cols >> 3) << 17);
       const int ctas = std::min(pp.n_items, dev.sms);
-      const bool is_max = pr.reduction == FCR_MAX;
-      if (pl.d_pad == 64)
-        e = is_max ? launch_onesweep<64, RED_MAX>(map_qc, map_k, pp, chunk_state, head_count, idesc_cols, copies, ctas, stream)
-                   : launch_onesweep<64, RED_SUM>(map_qc, map_k, pp, chunk_state, head_count, idesc_cols, copies, ctas, stream);
-      else
-        e = is_max ? launch_onesweep<128, RED_MAX>(map_qc, map_k, pp, chunk_state, head_count, idesc_cols, copies, ctas, stream)
-                   : launch_onesweep<128, RED_SUM>(map_qc, map_k, pp, chunk_state, head_count, idesc_cols, copies, ctas, stream);
-      if (e == cudaSuccess) {
-        trace_mark(1, stream);
-        trace_mark(2, stream);
-        return FCR_OK;
-      }
-      if (e != cudaErrorCooperativeLaunchTooLarge) return cuda_fail(e, "one-sweep kernel launch");
-      cudaGetLastError();  // clear it
-      fill(false);
+      rc = pr.reduction == FCR_MAX
+               ? launch_onesweep_d<RED_MAX>(pl.d_pad, map_qc, map_k, pp, chunk_state, counters, idesc_cols, copies, ctas, stream)
+               : launch_onesweep_d<RED_SUM>(pl.d_pad, map_qc, map_k, pp, chunk_state, counters, idesc_cols, copies, ctas, stream);
+      if (rc != FCR_OK) return rc;
+      trace_mark(1, stream);
+      trace_mark(2, stream);
+      return FCR_OK;
     }
     // the score cache is used when the caller's workspace has room for it
     const bool use_cache = pl.score_cache && (int64_t)workspace_bytes >= pl.workspace_bytes;

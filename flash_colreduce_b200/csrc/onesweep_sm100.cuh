@@ -3,17 +3,17 @@
 //
 // What bounds the shape is reading K: 2 * D bytes per key against 4 * M * D flops.  Two kernels read it
 // twice (a batch's K is far larger than the L2 cache).  Here a CTA alternates between the two passes on
-// small chunks of keys: segment 2n is the rows pass of its n-th chunk, segment 2n + 1 the columns pass of
-// its (n-1)-th, whose key tiles it asked for one segment pair earlier and which therefore come from the L2
+// small chunks of keys: record n is the rows pass of its n-th chunk, then the columns pass of
+// its (n-1)-th, whose key tiles it asked for one record earlier and which therefore come from the L2
 // (onesweep_chunks bounds the chunk for that).  The rows' chunk
 // states of a head are exchanged through global memory: the statistics warps merge the four warpgroups'
 // states of a chunk, publish them and count the chunk in a per-head counter; before a columns segment they
 // wait until all chunks of its head are counted and fold them, in chunk order, into the lse values.
 //
-// The CTAs wait on one another, so the launch is cooperative (all CTAs resident).  No cycle: item i is
-// chunk i % S of head i / S and belongs to CTA i % G, with S <= G the chunks of a head span at most two
-// consecutive segment pairs, a rows segment waits for no other CTA, and each CTA finishes the rows segment
-// n before its columns segment n - 1.
+// The CTAs wait on one another, but not for CTAs that have yet to start: the TMA warp draws the chunks from a ticket
+// counter and deals the records (OneSweepDealer, which has the argument), so that the call finishes on whatever SMs
+// are free.  Dealt round-robin to CTAs that all had to be resident (a cooperative launch), it could not even start
+// while a kernel of another stream held one SM.
 //
 // Measured (whole call, sustained): 16 x 32 heads, 64 x 16384, d = 128, fp16: 876 us in two sweeps, 640 in one;
 // 8 heads, 64 x 32768: 43 -> 27; one head, 64 x 60000: 85 -> 21 (few heads: the combination of many partial
@@ -37,13 +37,13 @@ constexpr int kOsMmaWarps = 2;  // take the tiles in turn: issuing one costs a w
 constexpr int kOsStatWarp = kKsMmaWarp + kOsMmaWarps;
 constexpr int kOsStatWarps = 4;
 constexpr int kOsThreads = (kOsStatWarp + kOsStatWarps) * 32;
-// Segment pairs between the two sweeps over a chunk.  Two hide the exchange no better (chunks of 5 tiles: 770
-// against 767 us) and keep twice the bytes in the L2 (chunks of 8: 778 against 680).
-constexpr int kOsLag = 1;
 constexpr int kOsLseBuffers = 4;    // chunks whose lse values may wait for their columns segment
 // Chunks whose warpgroup states may wait to be merged: one buffer per team of statistics warps, so that the uses of
 // a buffer are waited for by one team, in order.
 constexpr int kOsPartBuffers = 4;
+// Records announced to the other warps.  The TMA warp deals one ahead; the statistics warps may lag by the part buffers.
+constexpr int kOsRecords = 16;
+constexpr int kOsEnd = -2;  // the rows item of the last record
 constexpr int kOsChunk = 32;  // accumulator columns per tensor-memory load (736 threads: 80 registers)
 
 enum {
@@ -59,6 +59,8 @@ enum {
   ST_OS_WAIT_HEAD = 70,
   ST_OS_WAIT_LSE_EMPTY = 71,
   ST_OS_WAIT_LSE_FULL = 72,
+  ST_OS_WAIT_RECORD_EMPTY = 73,
+  ST_OS_WAIT_RECORD_FULL = 74,
 };
 
 template <int DPAD>
@@ -72,9 +74,11 @@ struct OneSweepSmem {
   static constexpr int off_part = off_ring + KR * kTileBytes;              // float2 [kOsPartBuffers][kKsBuffers][kTile]
   static constexpr int off_lse = off_part + kOsPartBuffers * kKsBuffers * kTile * 8;    // float [kOsLseBuffers][kTile]
   static constexpr int off_bars = off_lse + kOsLseBuffers * kTile * 4;
-  static constexpr int kNumBars = 4 + 2 * KR + 2 * kKsBuffers + 2 * kOsPartBuffers + 2 * kOsLseBuffers;
+  static constexpr int kNumBars = 4 + 2 * KR + 2 * kKsBuffers + 2 * kOsPartBuffers + 2 * kOsLseBuffers + 2 * kOsRecords;
   static constexpr int off_misc = off_bars + 8 * kNumBars;
-  static constexpr int kDynamicBytes = off_misc + 16;
+  static constexpr int off_records = off_misc + 16;              // int [kOsRecords][2]: rows item, columns item
+  static constexpr int off_held = off_records + 8 * kOsRecords;  // int [kOneSweepHeld], the dealer's
+  static constexpr int kDynamicBytes = off_held + 4 * kOneSweepHeld;
   static_assert(kDynamicBytes <= 232448, "exceeds the 227 KB shared memory of an sm_100 CTA");
 };
 
@@ -82,7 +86,7 @@ template <int DPAD, int RED>
 __global__ void __launch_bounds__(kOsThreads, 1)
 onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const PassParams p, float2* __restrict__ chunk_state, int* __restrict__ head_count,
-                const uint32_t idesc_cols, const int copies) {
+                int* __restrict__ ticket_count, const uint32_t idesc_cols, const int copies) {
   using L = OneSweepSmem<DPAD>;
   constexpr int KR = L::KR;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -105,15 +109,24 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   auto bar_part_empty = [&](uint32_t i) { return bar0 + 8u * (kTail + kOsPartBuffers + i); };
   auto bar_lse_full = [&](uint32_t i) { return bar0 + 8u * (kTail + 2 * kOsPartBuffers + i); };
   auto bar_lse_empty = [&](uint32_t i) { return bar0 + 8u * (kTail + 2 * kOsPartBuffers + kOsLseBuffers + i); };
+  auto bar_rec_full = [&](uint32_t i) { return bar0 + 8u * (kTail + 2 * kOsPartBuffers + 2 * kOsLseBuffers + i); };
+  auto bar_rec_empty = [&](uint32_t i) {
+    return bar0 + 8u * (kTail + 2 * kOsPartBuffers + 2 * kOsLseBuffers + kOsRecords + i);
+  };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + L::off_misc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::off_misc + 4);
   float2* const part_s = reinterpret_cast<float2*>(smem + L::off_part);
   float* const lse_all = reinterpret_cast<float*>(smem + L::off_lse);
+  volatile int* const records = reinterpret_cast<volatile int*>(smem + L::off_records);
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // warp-uniform for the compiler
   const int lane = (int)(threadIdx.x & 31);
   const int live_warps = (p.M + 31) >> 5;  // statistics warps (and 32-lane groups of a query tile) that hold a query
   const int copy_rows = kTile / copies;    // rows of one copy of the query tile
+
+  // the first ticket, asked for before the set-up so that its round trip passes meanwhile
+  int first_ticket = 0;
+  if (warp == kKsProducerWarp && lane == 0) first_ticket = atomicAdd(ticket_count, 1);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -136,6 +149,10 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       ptx::mbar_init(bar_tm_full(b), 1);
       ptx::mbar_init(bar_tm_empty(b), 4);
     }
+    for (int i = 0; i < kOsRecords; ++i) {
+      ptx::mbar_init(bar_rec_full(i), 1);
+      ptx::mbar_init(bar_rec_empty(i), kKsSoftmaxWarps + kOsMmaWarps + live_warps * copies);
+    }
     *abort_flag = 0;
     ptx::fence_mbar_init();
   }
@@ -154,19 +171,26 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   if (threadIdx.x == 0) ptx::grid_launch_dependents();
   if (p.clear_status && blockIdx.x == 0 && threadIdx.x < 4) p.status[threadIdx.x] = 0;
 
-  // Segment seg of this CTA: kind 0 = rows pass of chunk seg / 2, kind 1 = columns pass of chunk
-  // seg / 2 - 1 of the CTA's chunks blockIdx.x, blockIdx.x + G, ...  Every warp walks the same list.
+  // A record is the rows pass of one chunk (kind 0) and then the columns pass of another (kind 1), or one of them.
   const int S = p.n_split;
-  const int G = (int)gridDim.x;
-  const int n_chunks = (p.n_items - (int)blockIdx.x + G - 1) / G;
-  const int n_segs = 2 * (n_chunks + kOsLag);
-  struct Segment { int item, bh, sp, t_lo, t_hi; };
-  auto segment = [&](int seg, Segment& g) {
-    const int n = (seg >> 1) - (seg & 1) * kOsLag;
-    if (n < 0 || n >= n_chunks) return false;
-    g.item = (int)blockIdx.x + n * G;
-    keystream_item(S, p.key_tiles, g.item, g.bh, g.sp, g.t_lo, g.t_hi);
+  struct Record { int item[2]; };
+  struct Segment { int bh, sp, t_lo, t_hi; };
+  auto segment = [&](const Record& r, int kind, Segment& g) {
+    const int item = kind == 0 ? r.item[0] : r.item[1];
+    if (item < 0) return false;
+    keystream_item(S, p.key_tiles, item, g.bh, g.sp, g.t_lo, g.t_hi);
     return true;
+  };
+  // The n-th record, as the TMA warp announced it; false at the end, or when the wait for it expired (then not ok).
+  auto next_record = [&](uint32_t n, Record& r, bool& ok) {
+    const uint32_t i = n % kOsRecords;
+    ok = WAIT(bar_rec_full(i), (n / kOsRecords) & 1u, ST_OS_WAIT_RECORD_FULL);
+    if (!ok) return false;
+    r.item[0] = records[2 * i];
+    r.item[1] = records[2 * i + 1];
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive(bar_rec_empty(i));
+    return r.item[0] != kOsEnd;
   };
 
   if (warp == kKsProducerWarp) {
@@ -175,62 +199,91 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     // latter first (without the hint the large batch above takes 812 us, its second sweep missing half the time).
     const uint64_t keep = ptx::l2_policy_evict_normal(), drop = ptx::l2_policy_evict_first();
     uint32_t ring_seq = 0, q_seq[2] = {0, 0};
-    int cur_bh[2] = {-1, -1};
     bool ok = true;
-    for (int seg2 = 0; ok && seg2 < n_segs; seg2 += 2) {
+    // one pass over a chunk: its head's query tile (a head's chunks go to different CTAs), then its key tiles
+    auto load_segment = [&](const Segment& g, int kind) {
+      const int b = g.bh / p.H, h = g.bh - b * p.H;
+      if (!WAIT(bar_q_empty(kind), (q_seq[kind] & 1u) ^ 1u, ST_OS_WAIT_Q_EMPTY)) return false;
+      if (lane == 0) {
+        ptx::mbar_arrive_expect_tx(bar_q_full(kind), L::kTileBytes);
+        for (int c = 0; c < copies; ++c)
 #pragma unroll
-      for (int kind = 0; kind < 2; ++kind) {
-        Segment g;
-        if (!ok || !segment(seg2 + kind, g)) continue;
-        const int b = g.bh / p.H, h = g.bh - b * p.H;
-        if (g.bh != cur_bh[kind]) {
-          ok = WAIT(bar_q_empty(kind), (q_seq[kind] & 1u) ^ 1u, ST_OS_WAIT_Q_EMPTY);
-          if (!ok) continue;
-          if (lane == 0) {
-            ptx::mbar_arrive_expect_tx(bar_q_full(kind), L::kTileBytes);
-            for (int c = 0; c < copies; ++c)
-#pragma unroll
-              for (int hf = 0; hf < L::kHalves; ++hf)
-                ptx::tma_load_4d(s_q + kind * L::kTileBytes + hf * L::kHalfBytes + c * copy_rows * 128, &tmap_q,
-                                 bar_q_full(kind), hf * p.slab_elems, 0, h, b);
-          }
-          __syncwarp();
-          ++q_seq[kind];
-          cur_bh[kind] = g.bh;
-        }
-        for (int t = g.t_lo; t < g.t_hi; ++t, ++ring_seq) {
-          const uint32_t s = ring_seq % KR, ph = (ring_seq / KR) & 1u;
-          ok = WAIT(bar_ring_empty(s), ph ^ 1u, ST_OS_WAIT_RING_EMPTY);
-          if (!ok) break;
-          if (lane == 0) {
-            ptx::mbar_arrive_expect_tx(bar_ring_full(s), L::kTileBytes);
-#pragma unroll
-            for (int hf = 0; hf < L::kHalves; ++hf)
-              ptx::tma_load_4d_hint(s_ring + s * L::kTileBytes + hf * L::kHalfBytes, &tmap_k, bar_ring_full(s),
-                                    hf * p.slab_elems, t * kTile, h, b, kind == 0 ? keep : drop);
-          }
-          __syncwarp();
-        }
+          for (int hf = 0; hf < L::kHalves; ++hf)
+            ptx::tma_load_4d(s_q + kind * L::kTileBytes + hf * L::kHalfBytes + c * copy_rows * 128, &tmap_q,
+                             bar_q_full(kind), hf * p.slab_elems, 0, h, b);
       }
+      __syncwarp();
+      ++q_seq[kind];
+      for (int t = g.t_lo; t < g.t_hi; ++t, ++ring_seq) {
+        const uint32_t s = ring_seq % KR, ph = (ring_seq / KR) & 1u;
+        if (!WAIT(bar_ring_empty(s), ph ^ 1u, ST_OS_WAIT_RING_EMPTY)) return false;
+        if (lane == 0) {
+          ptx::mbar_arrive_expect_tx(bar_ring_full(s), L::kTileBytes);
+#pragma unroll
+          for (int hf = 0; hf < L::kHalves; ++hf)
+            ptx::tma_load_4d_hint(s_ring + s * L::kTileBytes + hf * L::kHalfBytes, &tmap_k, bar_ring_full(s),
+                                  hf * p.slab_elems, t * kTile, h, b, kind == 0 ? keep : drop);
+        }
+        __syncwarp();
+      }
+      return true;
+    };
+    uint32_t n = 0;  // records so far
+    OneSweepDealer dealer;
+    dealer.start(S, p.n_items, reinterpret_cast<int*>(smem + L::off_held), __shfl_sync(0xffffffffu, first_ticket, 0));
+    Record r;
+    auto announce = [&]() {
+      if (dealer.finished())
+        r.item[0] = kOsEnd;
+      else
+        dealer.deal(r.item[0], r.item[1]);
+      const uint32_t i = n % kOsRecords;
+      if (!WAIT(bar_rec_empty(i), ((n / kOsRecords) & 1u) ^ 1u, ST_OS_WAIT_RECORD_EMPTY)) return false;
+      if (lane == 0) {
+        records[2 * i] = r.item[0];
+        records[2 * i + 1] = r.item[1];
+        ptx::mbar_arrive(bar_rec_full(i));
+      }
+      __syncwarp();
+      ++n;
+      return true;
+    };
+    ok = announce();
+    while (ok && r.item[0] != kOsEnd) {
+      const bool draw = dealer.needs_ticket(), first = n == 1;
+      // Asked for here, needed after the rows pass's loads.  The first one waits until a tile has landed: by then every
+      // CTA of the launch has had its turn, and a chunk that an idle SM could have does not queue up behind another.
+      int ticket = 0;
+      if (draw && !first && lane == 0) ticket = atomicAdd(ticket_count, 1);
+      Segment g;
+      if (segment(r, 0, g)) ok = load_segment(g, 0);
+      if (!ok) break;
+      if (first) {
+        if (ring_seq <= KR) ok = WAIT(bar_ring_full(0), 0, ST_OS_WAIT_RING_FULL);  // (else a slot has been given back)
+        if (!ok) break;
+        if (draw && lane == 0) ticket = atomicAdd(ticket_count, 1);
+      }
+      const Record now = r;
+      if (draw) dealer.draw(__shfl_sync(0xffffffffu, ticket, 0));
+      ok = announce();
+      if (!ok) break;
+      if (segment(now, 1, g)) ok = load_segment(g, 1);
     }
   } else if (warp < kOsStatWarp && warp >= kKsMmaWarp) {
     // ------------------------------------------------------------ MMA warps
     const uint32_t my_turn = (uint32_t)(warp - kKsMmaWarp);
     uint32_t ring_seq = 0, q_seq[2] = {0, 0};
-    int cur_bh[2] = {-1, -1};
     bool ok = true;
-    for (int seg2 = 0; ok && seg2 < n_segs; seg2 += 2) {
+    Record r;
+    for (uint32_t n = 0; ok && next_record(n, r, ok); ++n) {
 #pragma unroll
       for (int kind = 0; kind < 2; ++kind) {
         Segment g;
-        if (!ok || !segment(seg2 + kind, g)) continue;
-        if (g.bh != cur_bh[kind]) {
-          ok = WAIT(bar_q_full(kind), q_seq[kind] & 1u, ST_OS_WAIT_Q_FULL);
-          if (!ok) continue;
-          ptx::tc_fence_after_sync();
-          ++q_seq[kind];
-          cur_bh[kind] = g.bh;
-        }
+        if (!ok || !segment(r, kind, g)) continue;
+        ok = WAIT(bar_q_full(kind), q_seq[kind] & 1u, ST_OS_WAIT_Q_FULL);
+        if (!ok) continue;
+        ptx::tc_fence_after_sync();
+        ++q_seq[kind];
         for (int t = g.t_lo; t < g.t_hi; ++t, ++ring_seq) {
           if (ring_seq % kOsMmaWarps != my_turn) continue;
           const uint32_t s = ring_seq % KR, ph = (ring_seq / KR) & 1u;
@@ -267,12 +320,9 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           __syncwarp();
         }
         if (!ok) continue;
-        // the last chunk of this head in a row: its query tile may be replaced once these MMAs retire
-        const int next_bh = (g.item + G < p.n_items) ? (g.item + G) / S : -1;
-        if (next_bh != g.bh) {
-          if (ptx::elect_one()) ptx::umma_commit(bar_q_empty(kind));
-          __syncwarp();
-        }
+        // the query tile may be replaced once these MMAs retire
+        if (ptx::elect_one()) ptx::umma_commit(bar_q_empty(kind));
+        __syncwarp();
       }
     }
     // The last commits cover every MMA issued by either warp: no asynchronous arrive is outstanding when the CTA retires.
@@ -286,36 +336,14 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const int team = (warp - kOsStatWarp) / team_warps, w = (warp - kOsStatWarp) % team_warps;
     const int i = w * 32 + lane;  // query
     bool ok = w < live_warps;
-    // Chunk n: publish its state as soon as its rows segment is folded, then fetch its head's lse values, a
-    // whole segment pair before the columns segment needs them.  (Waits of a chunk whose head ends in the next
-    // round of chunks are on CTAs of a smaller index whose own chunk does not: still no cycle.)
-    for (int n = team; ok && n < n_chunks; n += copies) {
+    // Of each record first the lse values of its columns pass, then the state of its rows pass: the fetch then starts as
+    // soon as the record before it is published, a whole rows pass before the columns pass needs the values.  (It waits
+    // for chunks of smaller tickets only, never for the record's own rows.)
+    uint32_t n_rows = 0, n_cols = 0;  // passes so far; the teams take them in turn
+    Record r;
+    for (uint32_t n = 0; ok && next_record(n, r, ok); ++n) {
       Segment g;
-      segment(2 * n, g);
-      const uint32_t pb = (uint32_t)n % kOsPartBuffers, pph = ((uint32_t)n / kOsPartBuffers) & 1u;
-      {
-        ok = WAIT(bar_part_full(pb), pph, ST_OS_WAIT_PART_FULL);
-        if (!ok) break;
-        // the four warpgroups' states of this chunk, in the order of their tiles
-        const float2* cell = part_s + pb * (kKsBuffers * kTile) + i;
-        float mx = -INFINITY, l = 0.f;
-        for (int c = 0; c < copies; ++c)
-#pragma unroll
-          for (int j = 0; j < kKsBuffers; ++j) mx = fmaxf(mx, cell[j * kTile + c * copy_rows].x);
-        for (int c = 0; c < copies; ++c)
-#pragma unroll
-          for (int j = 0; j < kKsBuffers; ++j) {
-            const float2 st = cell[j * kTile + c * copy_rows];
-            if (st.x != -INFINITY || st.y != 0.f) l = fmaf(st.y, exp2f(st.x - mx), l);
-          }
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(bar_part_empty(pb));
-        if (i < p.M) __stcg(chunk_state + ((size_t)g.sp * p.BH + g.bh) * p.m_pad + i, make_float2(mx, l));
-        __syncwarp();  // lane 0's release covers the stores of all lanes
-        if (lane == 0) ptx::red_release_add(head_count + (size_t)g.bh * kOsStatWarps + w, 1);
-        __syncwarp();
-      }
-      {
+      if (segment(r, 1, g) && (int)(n_cols++ % copies) == team) {
         // every chunk of the head has been counted by this warp of whichever CTA folded it
         if (lane == 0) {
           const int* count = head_count + (size_t)g.bh * kOsStatWarps + w;
@@ -361,12 +389,35 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
               if (v[u].x != -INFINITY || v[u].y != 0.f) l = fmaf(v[u].y, exp2f(v[u].x - mx), l);
           }
         }
-        const uint32_t lb = (uint32_t)n % kOsLseBuffers, lph = ((uint32_t)n / kOsLseBuffers) & 1u;
+        const uint32_t lb = (n_cols - 1) % kOsLseBuffers, lph = ((n_cols - 1) / kOsLseBuffers) & 1u;
         ok = WAIT(bar_lse_empty(lb), lph ^ 1u, ST_OS_WAIT_LSE_EMPTY);
         if (!ok) break;
         lse_all[lb * kTile + i] = i < p.M ? -(mx + log2f(l)) : 0.f;
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(bar_lse_full(lb));
+      }
+      if (segment(r, 0, g) && (int)(n_rows++ % copies) == team) {
+        const uint32_t pb = (n_rows - 1) % kOsPartBuffers, pph = ((n_rows - 1) / kOsPartBuffers) & 1u;
+        ok = WAIT(bar_part_full(pb), pph, ST_OS_WAIT_PART_FULL);
+        if (!ok) break;
+        // the four warpgroups' states of this chunk, in the order of their tiles
+        const float2* cell = part_s + pb * (kKsBuffers * kTile) + i;
+        float mx = -INFINITY, l = 0.f;
+        for (int c = 0; c < copies; ++c)
+#pragma unroll
+          for (int j = 0; j < kKsBuffers; ++j) mx = fmaxf(mx, cell[j * kTile + c * copy_rows].x);
+        for (int c = 0; c < copies; ++c)
+#pragma unroll
+          for (int j = 0; j < kKsBuffers; ++j) {
+            const float2 st = cell[j * kTile + c * copy_rows];
+            if (st.x != -INFINITY || st.y != 0.f) l = fmaf(st.y, exp2f(st.x - mx), l);
+          }
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(bar_part_empty(pb));
+        if (i < p.M) __stcg(chunk_state + ((size_t)g.sp * p.BH + g.bh) * p.m_pad + i, make_float2(mx, l));
+        __syncwarp();  // lane 0's release covers the stores of all lanes
+        if (lane == 0) ptx::red_release_add(head_count + (size_t)g.bh * kOsStatWarps + w, 1);
+        __syncwarp();
       }
     }
   } else {
@@ -382,103 +433,107 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const bool live = first_q < p.M;
     uint32_t seq = 0, n_rows = 0, n_cols = 0;  // tiles and segments so far
     bool ok = true;
-    for (int seg = 0; ok && seg < n_segs; ++seg) {
-      Segment g;
-      if (!segment(seg, g)) continue;
-      const int j0 = (int)((uint32_t)(wg - (int)seq) & (kKsBuffers - 1));  // my first tile within the chunk
-      const uint32_t seq0 = seq;
-      seq += (uint32_t)(g.t_hi - g.t_lo);
-      if ((seg & 1) == 0) {
-        const int mine = first_q + lane;  // query row
-        float m_run = -INFINITY, l_run = 0.f;
-        // keys j < valid_hi are attended by this query; tiles from mask_from on meet a mask edge
-        const int valid_hi = p.causal ? (int)hd_min((long long)p.N, (long long)mine + p.off + 1) : p.N;
-        int mask_from = p.N >> 7;
-        if (p.causal) mask_from = (int)hd_min((long long)mask_from, ((long long)p.off + 1) >> 7);
-        for (int t = g.t_lo + j0; t < g.t_hi; t += kKsBuffers) {
-          const uint32_t use = (seq0 + (uint32_t)(t - g.t_lo)) / kKsBuffers;
-          ok = WAIT(bar_tm_full(wg), use & 1u, ST_OS_WAIT_TMEM_FULL);
-          if (!ok) break;
-          if (!live) {
-            if (lane == 0) ptx::mbar_arrive(bar_tm_empty(wg));
-            __syncwarp();
-            continue;
-          }
-          ptx::tc_fence_after_sync();
-          const bool need_mask = t >= mask_from;
-          const int lim_hi = valid_hi - t * kTile - col0;
-          const int n_fold = copy_rows / kOsChunk;
-          uint32_t ra[kOsChunk];
-          for (int c = 0; c < n_fold; ++c) {
-            ptx::tmem_ld<kOsChunk>(taddr + col0 + c * kOsChunk, ra);
-            ptx::tmem_ld_wait<kOsChunk>(ra);
-            if (c + 1 == n_fold) {
-              ptx::tc_fence_before_sync();
-              __syncwarp();
+    Record r;
+    for (uint32_t n = 0; ok && next_record(n, r, ok); ++n) {
+#pragma unroll 1  // (unrolled, the sum reduction spills two of its 80 registers)
+      for (int kind = 0; kind < 2; ++kind) {
+        Segment g;
+        if (!ok || !segment(r, kind, g)) continue;
+        const int j0 = (int)((uint32_t)(wg - (int)seq) & (kKsBuffers - 1));  // my first tile within the chunk
+        const uint32_t seq0 = seq;
+        seq += (uint32_t)(g.t_hi - g.t_lo);
+        if (kind == 0) {
+          const int mine = first_q + lane;  // query row
+          float m_run = -INFINITY, l_run = 0.f;
+          // keys j < valid_hi are attended by this query; tiles from mask_from on meet a mask edge
+          const int valid_hi = p.causal ? (int)hd_min((long long)p.N, (long long)mine + p.off + 1) : p.N;
+          int mask_from = p.N >> 7;
+          if (p.causal) mask_from = (int)hd_min((long long)mask_from, ((long long)p.off + 1) >> 7);
+          for (int t = g.t_lo + j0; t < g.t_hi; t += kKsBuffers) {
+            const uint32_t use = (seq0 + (uint32_t)(t - g.t_lo)) / kKsBuffers;
+            ok = WAIT(bar_tm_full(wg), use & 1u, ST_OS_WAIT_TMEM_FULL);
+            if (!ok) break;
+            if (!live) {
               if (lane == 0) ptx::mbar_arrive(bar_tm_empty(wg));
+              __syncwarp();
+              continue;
             }
-            if (need_mask)
-              rows_chunk<true, kOsChunk>(ra, p.scale2, lim_hi - kOsChunk * c, m_run, l_run);
-            else
-              rows_chunk<false, kOsChunk>(ra, p.scale2, kOsChunk, m_run, l_run);
+            ptx::tc_fence_after_sync();
+            const bool need_mask = t >= mask_from;
+            const int lim_hi = valid_hi - t * kTile - col0;
+            const int n_fold = copy_rows / kOsChunk;
+            uint32_t ra[kOsChunk];
+            for (int c = 0; c < n_fold; ++c) {
+              ptx::tmem_ld<kOsChunk>(taddr + col0 + c * kOsChunk, ra);
+              ptx::tmem_ld_wait<kOsChunk>(ra);
+              if (c + 1 == n_fold) {
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(bar_tm_empty(wg));
+              }
+              if (need_mask)
+                rows_chunk<true, kOsChunk>(ra, p.scale2, lim_hi - kOsChunk * c, m_run, l_run);
+              else
+                rows_chunk<false, kOsChunk>(ra, p.scale2, kOsChunk, m_run, l_run);
+            }
           }
-        }
-        if (!ok) break;
-        const uint32_t pb = n_rows % kOsPartBuffers, pph = (n_rows / kOsPartBuffers) & 1u;
-        ++n_rows;
-        ok = WAIT(bar_part_empty(pb), pph ^ 1u, ST_OS_WAIT_PART_EMPTY);
-        if (!ok) break;
-        // a warpgroup without a tile in this chunk leaves (-inf, 0), which the merge skips
-        if (live) part_s[(pb * kKsBuffers + j0) * kTile + tid_wg] = make_float2(m_run, l_run);
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(bar_part_full(pb));
-      } else {
-        const uint32_t lb = n_cols % kOsLseBuffers, lph = (n_cols / kOsLseBuffers) & 1u;
-        ++n_cols;
-        ok = WAIT(bar_lse_full(lb), lph, ST_OS_WAIT_LSE_FULL);
-        if (!ok) break;
-        const float* lse_s = lse_all + lb * kTile;
-        const int n_fold = p.fold_cols / kChunkCols;  // only the chunks that hold a query
-        for (int t = g.t_lo + j0; t < g.t_hi; t += kKsBuffers) {
-          const uint32_t use = (seq0 + (uint32_t)(t - g.t_lo)) / kKsBuffers;
-          ok = WAIT(bar_tm_full(wg), use & 1u, ST_OS_WAIT_TMEM_FULL);
           if (!ok) break;
-          ptx::tc_fence_after_sync();
-          const int mine = t * kTile + tid_wg;  // key column
-          float acc[4];
+          const uint32_t pb = n_rows % kOsPartBuffers, pph = (n_rows / kOsPartBuffers) & 1u;
+          ++n_rows;
+          ok = WAIT(bar_part_empty(pb), pph ^ 1u, ST_OS_WAIT_PART_EMPTY);
+          if (!ok) break;
+          // a warpgroup without a tile in this chunk leaves (-inf, 0), which the merge skips
+          if (live) part_s[(pb * kKsBuffers + j0) * kTile + tid_wg] = make_float2(m_run, l_run);
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(bar_part_full(pb));
+        } else {
+          const uint32_t lb = n_cols % kOsLseBuffers, lph = (n_cols / kOsLseBuffers) & 1u;
+          ++n_cols;
+          ok = WAIT(bar_lse_full(lb), lph, ST_OS_WAIT_LSE_FULL);
+          if (!ok) break;
+          const float* lse_s = lse_all + lb * kTile;
+          const int n_fold = p.fold_cols / kChunkCols;  // only the chunks that hold a query
+          for (int t = g.t_lo + j0; t < g.t_hi; t += kKsBuffers) {
+            const uint32_t use = (seq0 + (uint32_t)(t - g.t_lo)) / kKsBuffers;
+            ok = WAIT(bar_tm_full(wg), use & 1u, ST_OS_WAIT_TMEM_FULL);
+            if (!ok) break;
+            ptx::tc_fence_after_sync();
+            const int mine = t * kTile + tid_wg;  // key column
+            float acc[4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) acc[u] = (RED == RED_MAX) ? -INFINITY : 0.f;
-          // queries max(mine - off, 0) <= i < M attend this key
-          const int valid_lo = p.causal ? max(mine - p.off, 0) : 0;
-          const bool need_mask = (p.M < p.fold_cols) || (p.causal && t * kTile + kTile - 1 - p.off > 0);
-          uint32_t ra[kChunkCols];
-          for (int c = 0; c < n_fold; ++c) {
-            ptx::tmem_ld<kChunkCols>(taddr + c * kChunkCols, ra);
-            ptx::tmem_ld_wait<kChunkCols>(ra);
-            if (c + 1 == n_fold) {
-              ptx::tc_fence_before_sync();
-              __syncwarp();
-              if (lane == 0) ptx::mbar_arrive(bar_tm_empty(wg));
+            for (int u = 0; u < 4; ++u) acc[u] = (RED == RED_MAX) ? -INFINITY : 0.f;
+            // queries max(mine - off, 0) <= i < M attend this key
+            const int valid_lo = p.causal ? max(mine - p.off, 0) : 0;
+            const bool need_mask = (p.M < p.fold_cols) || (p.causal && t * kTile + kTile - 1 - p.off > 0);
+            uint32_t ra[kChunkCols];
+            for (int c = 0; c < n_fold; ++c) {
+              ptx::tmem_ld<kChunkCols>(taddr + c * kChunkCols, ra);
+              ptx::tmem_ld_wait<kChunkCols>(ra);
+              if (c + 1 == n_fold) {
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(bar_tm_empty(wg));
+              }
+              if (need_mask)
+                cols_chunk<RED, true, kChunkCols>(ra, lse_s + kChunkCols * c, p.scale2, valid_lo - kChunkCols * c,
+                                                  p.M - kChunkCols * c, acc);
+              else
+                cols_chunk<RED, false, kChunkCols>(ra, lse_s + kChunkCols * c, p.scale2, 0, kChunkCols, acc);
             }
-            if (need_mask)
-              cols_chunk<RED, true, kChunkCols>(ra, lse_s + kChunkCols * c, p.scale2, valid_lo - kChunkCols * c,
-                                                p.M - kChunkCols * c, acc);
-            else
-              cols_chunk<RED, false, kChunkCols>(ra, lse_s + kChunkCols * c, p.scale2, 0, kChunkCols, acc);
+            if (mine < p.N) {
+              float v;
+              if (RED == RED_SUM)
+                v = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+              else
+                v = ptx::ex2(fmaxf(fmaxf(acc[0], acc[1]), fmaxf(acc[2], acc[3])));
+              if (p.mean_mode) v = v / mean_divisor(p, mine);
+              store_out(p.out, p.out_dtype, (size_t)g.bh * p.N + mine, v);
+            }
           }
-          if (mine < p.N) {
-            float v;
-            if (RED == RED_SUM)
-              v = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-            else
-              v = ptx::ex2(fmaxf(fmaxf(acc[0], acc[1]), fmaxf(acc[2], acc[3])));
-            if (p.mean_mode) v = v / mean_divisor(p, mine);
-            store_out(p.out, p.out_dtype, (size_t)g.bh * p.N + mine, v);
-          }
+          if (!ok) break;
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(bar_lse_empty(lb));  // done with these lse values
         }
-        if (!ok) break;
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(bar_lse_empty(lb));  // done with these lse values
       }
     }
   }

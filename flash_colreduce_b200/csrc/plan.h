@@ -22,6 +22,7 @@ constexpr int kTile = 128;            // rows per MMA tile (tensor-memory lanes)
 constexpr int kSubTiles = 2;          // stationary tiles a CTA owns
 constexpr int kBlockRows = kTile * kSubTiles;
 constexpr int kStatusWords = 256;
+constexpr int kOneSweepHeld = 256;    // chunks of one head a CTA of the one-sweep kernel can hold back
 
 // Geometry of one pass, shared by the host planner and the kernels.
 struct PassGeom {
@@ -55,6 +56,43 @@ FCR_HD void keystream_item(int S, int key_tiles, int item, int& bh, int& sp, int
   t_lo = (int)(((long long)key_tiles * sp) / S);
   t_hi = (int)(((long long)key_tiles * (sp + 1)) / S);
 }
+
+// What one CTA of the one-sweep kernel runs.  Its rows passes are the chunks whose indices it draws from a ticket
+// counter that all CTAs share (chunk i = part i % S of head i / S); it reduces the columns of a chunk of its own once
+// its newest ticket lies beyond the chunk's head.  The states that reduction waits for then all belong to smaller
+// tickets, drawn by CTAs that are running, and the smallest unfinished ticket waits for none: however few CTAs the GPU
+// has room for, they finish, and those that start later find no work.  (On an idle GPU a ticket is one chunk's rows
+// and the columns of the one before it.)
+struct OneSweepDealer {
+  int S, n_items;
+  int* held;      // [kOneSweepHeld] own chunks whose columns are still to come, oldest first
+  int head, tail; // of `held`
+  int ticket;     // newest ticket
+  int fresh;      // its rows have not been dealt
+  FCR_HD void start(int chunks_per_head, int items, int* storage, int first_ticket) {
+    S = chunks_per_head;
+    n_items = items;
+    held = storage;
+    head = tail = 0;
+    draw(first_ticket);
+  }
+  FCR_HD void draw(int t) {
+    ticket = t;
+    fresh = 1;
+  }
+  FCR_HD bool due() const {  // the oldest chunk's head ends before the newest ticket
+    return head != tail && (held[head % kOneSweepHeld] / S + 1) * S <= ticket;
+  }
+  FCR_HD bool finished() const { return ticket >= n_items && head == tail; }
+  FCR_HD bool needs_ticket() const { return !fresh && ticket < n_items && !due(); }
+  // The next rows pass and the next columns pass, in this order (-1: none).
+  FCR_HD void deal(int& rows, int& cols) {
+    rows = fresh && ticket < n_items ? ticket : -1;
+    cols = due() ? held[head++ % kOneSweepHeld] : -1;
+    if (rows >= 0) held[tail++ % kOneSweepHeld] = rows;
+    fresh = 0;
+  }
+};
 
 template <typename T>
 FCR_HD T hd_min(T a, T b) { return a < b ? a : b; }
@@ -167,8 +205,8 @@ inline int choose_splits(int64_t base_items, int64_t max_len_tiles, int num_sms)
 // chunk's tiles again one chunk later.  Unless all of K fits the L2 anyway, a chunk is at most 256 KB of K:
 // 16 x 32 heads, 64 x 16384, d = 128 took 1046 us with chunks of 3 tiles of 32 KB, 767 with 5, 665 with 8 and
 // 696 with 10 (two sweeps: 876), the small ones for the set-up of a chunk (about two tiles' time, the 2 in the
-// cost below), the large ones because the chunk has left the L2 before its second sweep.  S <= num_sms keeps
-// the waits between CTAs free of cycles.
+// cost below), the large ones because the chunk has left the L2 before its second sweep.  S <= num_sms, so that on
+// an idle GPU a CTA's next ticket lies beyond the head of its last one and each chunk is reduced one ticket later.
 // With rows of 128 bytes and more than 64 queries the folds bind, not the reading of K, and the second sweep
 // saves nothing: 256 heads, 128 x 8192, d = 64 took 158 us in two sweeps, 167 in one.  Only where K fits the
 // L2, whose problems are bound by the launches and the combination instead (4 heads, 128 x 65536: 56 -> 32 us).
@@ -181,7 +219,7 @@ inline int onesweep_chunks(const fcr_problem& p, const fcr_plan& pl, int num_sms
   if (!in_l2 && pl.d_pad == 64 && p.M > 64) return 0;
   int best = 0;
   int64_t best_cost = -1;
-  for (int64_t s = 1; s <= std::min<int64_t>(key_tiles, num_sms); ++s) {
+  for (int64_t s = 1; s <= std::min<int64_t>(key_tiles, std::min(num_sms, kOneSweepHeld)); ++s) {
     const int64_t tiles = ceil_div64(key_tiles, s);
     if (!in_l2 && tiles * tile_bytes > kOneSweepChunkBytes) continue;
     const int64_t cost = ceil_div64(BH * s, num_sms) * (tiles + 2);
@@ -195,8 +233,11 @@ inline int onesweep_chunks(const fcr_problem& p, const fcr_plan& pl, int num_sms
 // Copies of the query tile stacked in the 128 rows of an MMA: the spare rows repeat the queries, so that
 // the warps of the spare lanes fold their own share of a key tile's columns.
 inline int onesweep_copies(int M) { return M <= 32 ? 4 : (M <= 64 ? 2 : 1); }
-// Its scratch, the last region of the workspace: int[B*H][4] chunk counters, float2[S][B*H][m_pad] chunk states.
-inline int64_t onesweep_counter_bytes(const fcr_problem& p) { return align_up64((int64_t)p.B * p.H * 4 * 4, 256); }
+// Its scratch, the last region of the workspace: int[B*H][4] chunk counters and the ticket counter after them,
+// float2[S][B*H][m_pad] chunk states.
+inline int64_t onesweep_counter_bytes(const fcr_problem& p) {
+  return align_up64(((int64_t)p.B * p.H * 4 + 1) * 4, 256);
+}
 inline int64_t onesweep_bytes(const fcr_problem& p, const fcr_plan& pl, int num_sms) {
   const int64_t s = onesweep_chunks(p, pl, num_sms);
   return s == 0 ? 0 : onesweep_counter_bytes(p) + align_up64(s * p.B * p.H * pl.m_pad * 8, 256);

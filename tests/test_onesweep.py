@@ -2,6 +2,7 @@
 import ctypes as C
 import math
 import os
+import random
 import re
 import subprocess
 
@@ -27,6 +28,16 @@ extern "C" int chunks_of(int B, int H, int M, int N, int D, int causal, int dtyp
   out[8] = pl.off_part_l + 4ll * pl.row_splits * B * H * pl.m_pad;
   return fcr::onesweep_chunks(p, pl, sms);
 }
+extern "C" fcr::OneSweepDealer* dealer_new(int S, int n_items, int ticket) {
+  auto* d = new fcr::OneSweepDealer;
+  d->start(S, n_items, new int[fcr::kOneSweepHeld], ticket);
+  return d;
+}
+extern "C" void dealer_free(fcr::OneSweepDealer* d) { delete[] d->held; delete d; }
+extern "C" int dealer_finished(fcr::OneSweepDealer* d) { return d->finished(); }
+extern "C" int dealer_needs_ticket(fcr::OneSweepDealer* d) { return d->needs_ticket(); }
+extern "C" void dealer_draw(fcr::OneSweepDealer* d, int t) { d->draw(t); }
+extern "C" int dealer_deal(fcr::OneSweepDealer* d, int* out) { d->deal(out[0], out[1]); return d->tail - d->head; }
 extern "C" void item_of(int S, int key_tiles, int item, int* out) {
   fcr::keystream_item(S, key_tiles, item, out[0], out[1], out[2], out[3]);
 }
@@ -41,6 +52,9 @@ def planner(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", os.path.join(ROOT, "flash_colreduce_b200", "csrc"),
                     "-o", str(so), str(d / "harness.cpp")], check=True)
     lib = C.CDLL(str(so))
+    lib.dealer_new.restype = C.c_void_p
+    for name in ("dealer_free", "dealer_finished", "dealer_needs_ticket", "dealer_draw", "dealer_deal"):
+        getattr(lib, name).argtypes = [C.c_void_p] + {"dealer_draw": [C.c_int], "dealer_deal": [C.c_void_p]}.get(name, [])
 
     def plan(b, h, m, n, d, causal=1, dtype=0, sms=148):
         out = (C.c_longlong * 9)()
@@ -51,61 +65,166 @@ def planner(tmp_path_factory):
         lib.item_of(s, tiles, i, out)
         return tuple(out)
 
-    return plan, item
+    return plan, item, lib
 
 
-@pytest.mark.parametrize("b,h,m,n,sms", [(1, 1, 17, 1024, 148), (1, 1, 128, 90000, 148), (1, 1, 64, 70000, 3), (1, 3, 100, 9000, 7),
-                                         (16, 32, 64, 16384, 148), (1, 32, 128, 4096, 148), (2, 75, 33, 1027, 148), (1, 2, 40, 2000, 1), (2, 75, 32, 6000, 148),
-                                         (1, 40, 40, 13000, 100)])
-def test_schedule_covers_the_keys_and_never_waits_in_a_circle(planner, b, h, m, n, sms):
-    """Walks every CTA as the kernel does: its folding warps take rows segment n, then columns segment n - 1 (which
-    needs the lse values of that chunk); a team of statistics warps publishes chunk n once it is folded, then fetches
-    its lse values (which needs every chunk of the head published).  All must reach their end."""
-    plan, item = planner
+class _Cta:
+    """One CTA of the kernel as agents that wait for one another: the TMA warp (deals records, fills the ring), the folding
+    warps (with the MMA warps: a tile's slot is free once it is folded, which is later than in the kernel) and the teams of
+    statistics warps.  Every agent is a generator that yields the condition it waits for."""
+
+    def __init__(self, sim):
+        self.sim, self.loaded, self.folded, self.records = sim, 0, 0, []
+        self.folded_seg = [0, 0]             # rows and columns passes folded
+        self.loaded_seg = [0, 0]
+        self.parts_full, self.parts_read = 0, set()
+        self.lse_full, self.lse_done = set(), 0
+        self.agents = [self.tma(), self.fold()] + [self.stat(t) for t in range(sim.copies)]
+        self.read = {x: 0 for x in range(1 + sim.copies)}  # records read: by the folding warps, by each team
+
+    def segment(self, item, kind):
+        _, _, lo, hi = self.sim.item(self.sim.S, self.sim.tiles, item)
+        yield lambda: self.folded_seg[kind] >= self.loaded_seg[kind]  # the query tile of this kind is free
+        self.loaded_seg[kind] += 1
+        for _ in range(lo, hi):
+            yield lambda: self.loaded - self.folded < self.sim.ring
+            self.loaded += 1
+
+    def tma(self):
+        sim, out = self.sim, (C.c_int * 2)()
+        d = sim.lib.dealer_new(sim.S, sim.items, sim.draw())
+
+        def announce():
+            if sim.lib.dealer_finished(d):
+                rec = None
+            else:
+                held = sim.lib.dealer_deal(d, out)
+                assert held <= sim.S
+                rec = (out[0], out[1])
+                assert rec != (-1, -1)
+            self.records.append(rec)
+            return rec
+
+        rec, first = announce(), True
+        while rec is not None:
+            need = sim.lib.dealer_needs_ticket(d)
+            ticket = sim.draw() if need and not first else None
+            if rec[0] >= 0:
+                yield from self.segment(rec[0], 0)
+            if need:
+                sim.lib.dealer_draw(d, sim.draw() if first else ticket)
+            yield lambda: len(self.records) - min(self.read.values()) < 16
+            cols, rec, first = rec[1], announce(), False
+            if cols >= 0:
+                yield from self.segment(cols, 1)
+        sim.lib.dealer_free(d)
+
+    def next_record(self, reader):
+        yield lambda: len(self.records) > self.read[reader]
+        self.read[reader] += 1
+        return self.records[self.read[reader] - 1]
+
+    def fold(self):
+        n_rows = n_cols = 0
+        while (rec := (yield from self.next_record(0))) is not None:
+            for kind in (0, 1):
+                if rec[kind] < 0:
+                    continue
+                head, _, lo, hi = self.sim.item(self.sim.S, self.sim.tiles, rec[kind])
+                if kind == 1:
+                    yield lambda: n_cols in self.lse_full
+                    assert self.sim.counted[head] == self.sim.S
+                for _ in range(lo, hi):
+                    yield lambda: self.loaded > self.folded
+                    self.folded += 1
+                self.folded_seg[kind] += 1
+                self.sim.swept[kind].append(rec[kind])
+                if kind == 0:
+                    yield lambda: n_rows < 4 or n_rows - 4 in self.parts_read
+                    n_rows += 1
+                    self.parts_full = n_rows
+                else:
+                    n_cols += 1
+                    self.lse_done = n_cols
+
+    def stat(self, team):
+        sim, n_rows, n_cols = self.sim, 0, 0
+        while (rec := (yield from self.next_record(1 + team))) is not None:
+            if rec[1] >= 0:
+                if n_cols % sim.copies == team:
+                    head = rec[1] // sim.S
+                    yield lambda: sim.counted[head] == sim.S
+                    yield lambda: n_cols < 4 or self.lse_done > n_cols - 4
+                    self.lse_full.add(n_cols)
+                n_cols += 1
+            if rec[0] >= 0:
+                if n_rows % sim.copies == team:
+                    yield lambda: self.parts_full > n_rows
+                    self.parts_read.add(n_rows)
+                    sim.counted[rec[0] // sim.S] += 1
+                n_rows += 1
+
+
+class _Sim:
+    def __init__(self, lib, item, S, tiles, heads, m, ring, seed):
+        self.lib, self.item, self.S, self.tiles, self.items, self.ring = lib, item, S, tiles, heads * S, ring
+        self.copies = 4 if m <= 32 else 2 if m <= 64 else 1
+        self.counted, self.swept, self.tickets = [0] * heads, ([], []), 0
+        self.rng = random.Random(seed)
+
+    def draw(self):
+        self.tickets += 1
+        return self.tickets - 1
+
+    def run(self, grid, room):
+        """`grid` CTAs, of which `room` run at a time: the next one starts when one has ended."""
+        live, started = [], 0
+        while started < grid or live:
+            while started < grid and len(live) < room:
+                live.append([[g, None] for g in _Cta(self).agents])
+                started += 1
+            moved = False
+            self.rng.shuffle(live)
+            for cta in live:
+                for agent in list(cta):
+                    steps = 0
+                    while agent[1] is None or agent[1]():
+                        moved, steps = True, steps + 1
+                        try:
+                            agent[1] = next(agent[0])
+                        except StopIteration:
+                            cta.remove(agent)
+                            break
+                        if steps > self.rng.randrange(1, 40):
+                            break
+            if any(not cta for cta in live):
+                live = [cta for cta in live if cta]
+                moved = True
+            assert moved, "CTAs wait for good"
+
+
+@pytest.mark.parametrize("b,h,m,n,sms,room", [(1, 1, 17, 1024, 148, 148), (1, 1, 128, 90000, 148, 148), (1, 1, 128, 90000, 148, 1),
+                                              (1, 1, 64, 70000, 3, 3), (1, 3, 100, 9000, 7, 7), (1, 3, 100, 9000, 7, 2),
+                                              (4, 32, 64, 16384, 148, 148), (1, 32, 64, 16384, 148, 147), (1, 32, 64, 16384, 148, 1),
+                                              (1, 32, 128, 4096, 148, 148), (1, 32, 128, 4096, 148, 100), (1, 32, 128, 4096, 148, 1),
+                                              (2, 75, 33, 1027, 148, 148), (1, 2, 40, 2000, 1, 1), (2, 75, 32, 6000, 148, 148),
+                                              (2, 75, 32, 6000, 148, 5), (1, 40, 40, 13000, 100, 100), (1, 8, 64, 32768, 148, 3)])
+def test_every_chunk_is_swept_twice_however_few_ctas_run(planner, b, h, m, n, sms, room):
+    """A call finishes on the SMs that are free: with room for one CTA, for some or for all of the grid, whoever draws the
+    tickets first, no CTA waits for one that has not started, and each chunk has its rows and its columns pass once."""
+    plan, item, lib = planner
     S, info = plan(b, h, m, n, 128, sms=sms)
-    tiles, bh = info[3], b * h
+    tiles, heads = info[3], b * h
     assert 1 <= S <= min(tiles, sms)
-    items, G = bh * S, min(bh * S, sms)
     seen = {}
-    for i in range(items):
+    for i in range(heads * S):
         head, sp, lo, hi = item(S, tiles, i)
         assert head == i // S and sp == i % S and lo < hi
         seen.setdefault(head, []).extend(range(lo, hi))
-    assert all(seen[x] == list(range(tiles)) for x in range(bh))
-    chunks = [(items - c + G - 1) // G for c in range(G)]
-    copies, lag, buffers = (4 if m <= 32 else 2 if m <= 64 else 1), 1, 4
-    fold, counted, published, fetched = [0] * G, [0] * bh, [set() for _ in range(G)], [set() for _ in range(G)]
-    stat = [[0] * copies for _ in range(G)]  # steps done by each team: even ones publish a chunk, odd ones fetch
-    moved = True
-    while moved:
-        moved = False
-        for c in range(G):
-            for team in range(copies):
-                while team + copies * (stat[c][team] >> 1) < chunks[c]:
-                    n = team + copies * (stat[c][team] >> 1)
-                    head = (c + n * G) // S
-                    if stat[c][team] & 1:
-                        if counted[head] < S or (n >= buffers and fold[c] < 2 * (n - buffers + lag) + 2):
-                            break
-                        fetched[c].add(n)
-                    else:
-                        if fold[c] < 2 * n + 1:
-                            break
-                        published[c].add(n)
-                        counted[head] += 1
-                    stat[c][team] += 1
-                    moved = True
-            while fold[c] < 2 * (chunks[c] + lag):
-                n = (fold[c] >> 1) - (fold[c] & 1) * lag
-                if 0 <= n < chunks[c]:
-                    if fold[c] & 1:
-                        if n not in fetched[c]:
-                            break
-                    elif n >= buffers and n - buffers not in published[c]:
-                        break
-                fold[c] += 1
-                moved = True
-    assert all(fold[c] == 2 * (chunks[c] + lag) and len(fetched[c]) == chunks[c] for c in range(G)), "a CTA waits for good"
+    assert all(seen[x] == list(range(tiles)) for x in range(heads))
+    sim = _Sim(lib, item, S, tiles, heads, m, ring=4, seed=n)
+    sim.run(min(heads * S, sms), room)
+    assert sorted(sim.swept[0]) == sorted(sim.swept[1]) == list(range(heads * S))
 
 
 def test_the_exchange_orders_the_memory_of_all_lanes():
@@ -120,7 +239,7 @@ def test_the_exchange_orders_the_memory_of_all_lanes():
 
 
 def test_which_shapes_take_it_and_where_its_scratch_lies(planner):
-    plan, _ = planner
+    plan, _, _ = planner
     for m, n, d, dtype, takes in [(17, 1024, 128, 0, True), (128, 1024, 64, 0, True), (64, 4096, 80, 1, True), (64, 4096, 64, 2, True),
                                   (16, 4096, 128, 0, False),   # score cache
                                   (64, 4096, 129, 0, False), (64, 4096, 72, 2, False),  # rows beyond 256 bytes
@@ -202,7 +321,7 @@ def test_one_sweep_under_graph_capture_and_on_two_streams():
         s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
         torch.cuda.synchronize()
         got = []
-        for _ in range(20):  # cooperative launches of two streams wait for one another, never inside one another
+        for _ in range(20):  # blocks of the one call start as blocks of the other end
             for s in (s1, s2):
                 with torch.cuda.stream(s):
                     got.append(flash_colreduce(q, k, "sum", is_causal=True))
@@ -221,6 +340,43 @@ def test_one_sweep_under_graph_capture_and_on_two_streams():
             os.environ.pop("FCR_DEBUG_SYNC", None)
         else:
             os.environ["FCR_DEBUG_SYNC"] = old
+
+
+@pytest.mark.gpu
+def test_one_sweep_finishes_while_another_kernel_holds_an_sm():
+    """A kernel of another stream (one block that waits for a load left out on purpose until its bound of about 0.2 s runs
+    out) holds an SM that the call's grid would fill: the call ends on the others, with the same result."""
+    from flash_colreduce_b200 import _native as nat
+
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(9)
+    q = torch.randn(1, 32, 128, 128, generator=g, device=dev, dtype=torch.float16)
+    k = torch.randn(1, 32, 4096, 128, generator=g, device=dev, dtype=torch.float16)
+    x = torch.randn(1, 1, 128, 64, generator=g, device=dev, dtype=torch.float16)
+    out, launches, _, pr = _call(nat, q, k, "sum", True, 0.09)
+    assert launches == 1
+    one = nat.make_problem(1, 1, 128, 128, 64, x.stride(), x.stride(), nat.FCR_F16, nat.FCR_SUM, False, 0.125)
+    pl = nat.plan(one, 0)
+    assert pl.row_ctas == 1
+    ws = torch.empty(int(pl.workspace_bytes), dtype=torch.uint8, device=dev)
+    small = torch.empty(1, 1, 128, dtype=torch.float32, device=dev)
+    holder, other, held = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.Event()
+    torch.cuda.synchronize()
+    nat.check(nat.lib.fcr_self_test_hooks(400_000_000, 0), "fcr_self_test_hooks")
+    try:
+        nat.check(nat.lib.fcr_colreduce(C.byref(one), x.data_ptr(), x.data_ptr(), small.data_ptr(), nat.FCR_F32, ws.data_ptr(),
+                                        ws.numel(), holder.cuda_stream), "fcr_colreduce")
+    finally:
+        nat.check(nat.lib.fcr_self_test_hooks(0, -1), "fcr_self_test_hooks")
+    held.record(holder)
+    with torch.cuda.stream(other):
+        got, _, _, _ = _call(nat, q, k, "sum", True, 0.09)  # waits for its own stream
+        still_held = not held.query()
+    torch.cuda.synchronize()
+    code = C.c_int32(0)
+    assert nat.lib.fcr_poll_device_status(C.byref(code)) == nat.FCR_ERR_DEVICE_TIMEOUT  # the holder's report
+    assert still_held, "the call waited for the other kernel's SM"
+    assert torch.equal(got, out)
 
 
 @pytest.mark.gpu
