@@ -153,7 +153,8 @@ keystream_kernel(const __grid_constant__ CUtensorMap tmap_q,
         const uint32_t s = ring_seq % KR, ph = (ring_seq / KR) & 1u;
         ok = WAIT(bar_ring_empty(s), ph ^ 1u, ST_KS_WAIT_RING_EMPTY);
         if (!ok) break;
-        if (lane == 0) {
+        const bool left_out = blockIdx.x == 0 && (int)ring_seq == p.skip_ring_load;  // self-test of the bounded waits
+        if (lane == 0 && !left_out) {
           ptx::mbar_arrive_expect_tx(bar_ring_full(s), L::kTileBytes);
 #pragma unroll
           for (int hf = 0; hf < L::kHalves; ++hf)

@@ -217,7 +217,8 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       for (int t = g.t_lo; t < g.t_hi; ++t, ++ring_seq) {
         const uint32_t s = ring_seq % KR, ph = (ring_seq / KR) & 1u;
         if (!WAIT(bar_ring_empty(s), ph ^ 1u, ST_OS_WAIT_RING_EMPTY)) return false;
-        if (lane == 0) {
+        const bool left_out = blockIdx.x == 0 && (int)ring_seq == p.skip_ring_load;  // self-test of the bounded waits
+        if (lane == 0 && !left_out) {
           ptx::mbar_arrive_expect_tx(bar_ring_full(s), L::kTileBytes);
 #pragma unroll
           for (int hf = 0; hf < L::kHalves; ++hf)

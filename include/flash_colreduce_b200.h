@@ -321,12 +321,11 @@ int64_t fcr_launch_count(void);
  * Self-test of the bounded waits, for the calling thread's later
  * fcr_colreduce calls: `wait_limit_cycles` > 0 replaces the one-second bound
  * of every device-side wait (in SM clock cycles), and `skip_ring_load` >= 0
- * makes the first CTA of each pass kernel leave out its skip_ring_load-th
- * streamed-tile load, so that the waits on that tile expire: the kernels then
+ * makes the first CTA of each kernel that streams tiles leave out its
+ * skip_ring_load-th streamed-tile load, so that the waits on that tile expire: the kernels then
  * give up in an orderly way (no trap, no fault; tensor memory is released) and
  * the call's failure is reported as described at fcr_colreduce.  (0, -1)
- * restores normal operation.  The decode (key-streaming) kernels ignore
- * skip_ring_load.
+ * restores normal operation.
  */
 int fcr_self_test_hooks(int64_t wait_limit_cycles, int32_t skip_ring_load);
 

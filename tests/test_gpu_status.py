@@ -1,7 +1,7 @@
 """A device-side wait that runs out is reported to the host (needs a B200).
 
 The failure is made without faulting anything: a self-test hook makes the first
-CTA of each pass kernel leave out one streamed-tile load (nothing is in flight
+CTA of each kernel leave out one streamed-tile load (nothing is in flight
 for that slot) and shortens the bound of every device-side wait to about a
 millisecond.  The waits on the missing tile then expire, every warp of that CTA
 leaves through the kernel's normal give-up path (tensor memory released), the
@@ -115,3 +115,38 @@ def test_status_words_in_the_workspace_tell_the_same_story():
     assert code.value in (ST_WAIT_RING_FULL, ST_WAIT_TMEM_FULL)
     # that read also took the report out of the mailbox
     assert nat.lib.fcr_poll_device_status(C.byref(code)) == nat.FCR_OK
+
+
+# the decode shapes: key streaming with a score cache, key streaming with two sweeps (512-byte rows), one sweep with one
+# chunk per CTA, with several, with four teams of statistics warps and with one
+DECODE = [(4, 24, 8192, 128), (64, 24, 8192, 256), (64, 24, 8192, 128), (40, 150, 8192, 128), (20, 60, 4096, 64), (128, 32, 4096, 128)]
+
+
+@pytest.mark.parametrize("m,heads,n,d", DECODE)
+@pytest.mark.parametrize("skip", [0, 3])
+def test_expired_wait_in_the_decode_kernels(no_debug_sync, m, heads, n, d, skip):
+    """The CTA whose load is missing gives up, and so do the CTAs that wait for its chunk states; the call returns, reports
+    itself once, and the next call is right."""
+    from flash_colreduce_b200 import _native as nat
+    from flash_colreduce_b200 import flash_colreduce
+
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(m)
+    q = torch.randn(1, heads, m, d, generator=g).half()
+    k = torch.randn(1, heads, n, d, generator=g).half()
+    qd, kd = q.to(dev), k.to(dev)
+    before = flash_colreduce(qd, kd, "sum", is_causal=True)
+    torch.cuda.synchronize()
+    nat.check(nat.lib.fcr_self_test_hooks(2_000_000, skip), "fcr_self_test_hooks")
+    try:
+        flash_colreduce(qd, kd, "sum", is_causal=True)
+    finally:
+        nat.check(nat.lib.fcr_self_test_hooks(0, -1), "fcr_self_test_hooks")
+    torch.cuda.synchronize()
+    code = C.c_int32(-1)
+    assert nat.lib.fcr_poll_device_status(C.byref(code)) == nat.FCR_ERR_DEVICE_TIMEOUT
+    assert 50 < code.value < 80 and "bounded wait" in nat.last_error()
+    assert nat.lib.fcr_poll_device_status(C.byref(code)) == nat.FCR_OK
+    after = flash_colreduce(qd, kd, "sum", is_causal=True)
+    assert torch.equal(before, after)
+    assert_parity(after[:, :2], oracle_colreduce(q[:, :2], k[:, :2], "sum", True), "sum", extra_rtol=2.0 ** -11)
