@@ -117,7 +117,7 @@ struct PassParams : PassGeom {
   int div_M, div_N, div_c;
   int* status;
   int* host_status;       // the device's status mailbox in mapped host memory (null: none)
-  long long wait_limit;   // bound of every device-side wait, in clock64 cycles
+  long long wait_limit;   // bound of a device-side wait, in clock64 cycles (wait_bar: once to three times)
   int skip_ring_load;     // self-test: CTA 0's TMA warp leaves out this ring load (-1: none)
   int* sched_counter;  // zero at launch; hands out work items beyond the first gridDim.x (null: round-robin)
   int clear_status;    // 1: this kernel clears status words 0-3 itself (no memset ran before it)
@@ -186,8 +186,11 @@ struct SmemLayout {
 // hint), so a waiting warp polls.  Letting the waiting warps sleep between polls was measured
 // (100 ns to 1 us for the TMA and MMA warps, 50 and 200 ns for the fold warps): no timing changed by
 // more than the run-to-run noise, so they simply poll.
+// `bounds` is the wait's limit in units of PassParams::wait_limit: 1 for a wait on loads or products, which is where a
+// failure shows first; 2 or 3 for a wait on warps or blocks that themselves wait (the TMA warp's, for slots that its
+// consumers give back), so that it expires later and the status names the wait at the root.
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                         const PassParams& p, int code) {
+                                         const PassParams& p, int code, int bounds) {
   if (ptx::mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   uint32_t spins = 0;
@@ -195,9 +198,7 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
     if (ptx::mbar_try_wait(bar, parity)) return true;
     if ((++spins & 7u) == 0) {
       if (*abort_flag) return false;
-      // The TMA warp waits for slots that its consumers give back, so a consumer that is stuck makes it wait
-      // too, a few hundred cycles later: twice the bound for it, and the status names the wait at the root.
-      if (clock64() - t0 > (code < ST_WAIT_STAT_FULL ? 2 : 1) * p.wait_limit) {
+      if (clock64() - t0 > bounds * p.wait_limit) {
         *abort_flag = 1;
         report_status(p, code, (int)parity);
         return false;
@@ -207,10 +208,12 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
 }
 // Same, with a warp-uniform result so that .sync.aligned instructions that
 // follow are executed by all 32 lanes or by none.
-#define WAIT(bar, par, code) wait_bar_warp(bar, par, abort_flag, p, code)
-__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity,
-                                              volatile int* abort_flag, const PassParams& p, int code) {
-  const bool ok = wait_bar(bar, parity, abort_flag, p, code);
+#define WAIT(bar, par, code) wait_bar_warp(bar, par, abort_flag, p, code, 1)
+#define WAIT_BEHIND(bar, par, code) wait_bar_warp(bar, par, abort_flag, p, code, 2)
+#define WAIT_BEHIND_PEERS(bar, par, code) wait_bar_warp(bar, par, abort_flag, p, code, 3)
+__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                              const PassParams& p, int code, int bounds) {
+  const bool ok = wait_bar(bar, parity, abort_flag, p, code, bounds);
   return __all_sync(0xffffffffu, ok);
 }
 
@@ -360,7 +363,7 @@ pass_kernel(const __grid_constant__ CUtensorMap tmap_stat,
     auto load_stationary = [&](const Item& g, uint32_t seq) {
       const int b = g.bh / p.H, h = g.bh - b * p.H;
       const uint32_t ks = seq % KS, kph = (seq / KS) & 1u;
-      if (!WAIT(bar_stat_empty(ks), kph ^ 1u, ST_WAIT_STAT_EMPTY)) return false;
+      if (!WAIT_BEHIND(bar_stat_empty(ks), kph ^ 1u, ST_WAIT_STAT_EMPTY)) return false;
       if (lane == 0) {
         ptx::mbar_arrive_expect_tx(bar_stat_full(ks), kSubTiles * L::kTileBytes);
 #pragma unroll
@@ -394,7 +397,7 @@ pass_kernel(const __grid_constant__ CUtensorMap tmap_stat,
     if (kAhead && g.bh >= 0) ok = load_stationary(g, 0);
     for (; ok; ++item_seq) {
       const uint32_t si = item_seq % KI, sph = (item_seq / KI) & 1u;
-      ok = WAIT(bar_sched_empty(si), sph ^ 1u, ST_WAIT_SCHED_EMPTY);
+      ok = WAIT_BEHIND(bar_sched_empty(si), sph ^ 1u, ST_WAIT_SCHED_EMPTY);
       if (!ok) break;
       const bool last = g.bh < 0;
       if (lane == 0) {
@@ -436,7 +439,7 @@ pass_kernel(const __grid_constant__ CUtensorMap tmap_stat,
 #pragma unroll
         for (int piece = 0; piece < L::kPieces; ++piece, ++ring_seq) {
           const uint32_t s = ring_seq % KR, ph = (ring_seq / KR) & 1u;
-          ok = WAIT(bar_ring_empty(s), ph ^ 1u, ST_WAIT_RING_EMPTY);
+          ok = WAIT_BEHIND(bar_ring_empty(s), ph ^ 1u, ST_WAIT_RING_EMPTY);
           if (!ok) break;
           // self-test of the bounded waits: one load of CTA 0 is never requested (nothing is in
           // flight for its slot), so the consumers' waits on it run into their limit
@@ -454,7 +457,7 @@ pass_kernel(const __grid_constant__ CUtensorMap tmap_stat,
         if (!ok) break;
         if (PHASE == PH_COLS) {  // the tile's lse values, into their own ring
           const uint32_t sl = tile_seq % KL, lph = (tile_seq / KL) & 1u;
-          ok = WAIT(bar_lse_empty(sl), lph ^ 1u, ST_WAIT_LSE_EMPTY);
+          ok = WAIT_BEHIND(bar_lse_empty(sl), lph ^ 1u, ST_WAIT_LSE_EMPTY);
           if (!ok) break;
           if (lane == 0) {
             ptx::mbar_arrive_expect_tx(bar_lse_full(sl), L::kLseBytes);

@@ -134,7 +134,7 @@ keystream_kernel(const __grid_constant__ CUtensorMap tmap_q,
       keystream_item(S, p.key_tiles, item, bh, sp, t_lo, t_hi);
       const int b = bh / p.H, h = bh - b * p.H;
       if (bh != cur_bh) {
-        ok = WAIT(bar_q_empty, (q_seq & 1u) ^ 1u, ST_KS_WAIT_Q_EMPTY);
+        ok = WAIT_BEHIND(bar_q_empty, (q_seq & 1u) ^ 1u, ST_KS_WAIT_Q_EMPTY);
         if (!ok) break;
         if (lane == 0) {
           ptx::mbar_arrive_expect_tx(bar_q_full,
@@ -151,7 +151,7 @@ keystream_kernel(const __grid_constant__ CUtensorMap tmap_q,
       }
       for (int t = t_lo; t < t_hi; ++t, ++ring_seq) {
         const uint32_t s = ring_seq % KR, ph = (ring_seq / KR) & 1u;
-        ok = WAIT(bar_ring_empty(s), ph ^ 1u, ST_KS_WAIT_RING_EMPTY);
+        ok = WAIT_BEHIND(bar_ring_empty(s), ph ^ 1u, ST_KS_WAIT_RING_EMPTY);
         if (!ok) break;
         const bool left_out = blockIdx.x == 0 && (int)ring_seq == p.skip_ring_load;  // self-test of the bounded waits
         if (lane == 0 && !left_out) {

@@ -46,6 +46,8 @@ constexpr int kOsRecords = 16;
 constexpr int kOsEnd = -2;  // the rows item of the last record
 constexpr int kOsChunk = 32;  // accumulator columns per tensor-memory load (736 threads: 80 registers)
 
+// A missing tile shows first in its own CTA (bound 1: Q_FULL, RING_FULL, TMEM_FULL, DRAIN), then in the CTAs that wait for
+// its chunk's state (HEAD: 2), last in the warps that wait behind those (3).
 enum {
   ST_OS_WAIT_Q_EMPTY = 61,
   ST_OS_WAIT_RING_EMPTY = 62,
@@ -184,7 +186,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   // The n-th record, as the TMA warp announced it; false at the end, or when the wait for it expired (then not ok).
   auto next_record = [&](uint32_t n, Record& r, bool& ok) {
     const uint32_t i = n % kOsRecords;
-    ok = WAIT(bar_rec_full(i), (n / kOsRecords) & 1u, ST_OS_WAIT_RECORD_FULL);
+    ok = WAIT_BEHIND_PEERS(bar_rec_full(i), (n / kOsRecords) & 1u, ST_OS_WAIT_RECORD_FULL);
     if (!ok) return false;
     r.item[0] = records[2 * i];
     r.item[1] = records[2 * i + 1];
@@ -203,7 +205,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     // one pass over a chunk: its head's query tile (a head's chunks go to different CTAs), then its key tiles
     auto load_segment = [&](const Segment& g, int kind) {
       const int b = g.bh / p.H, h = g.bh - b * p.H;
-      if (!WAIT(bar_q_empty(kind), (q_seq[kind] & 1u) ^ 1u, ST_OS_WAIT_Q_EMPTY)) return false;
+      if (!WAIT_BEHIND_PEERS(bar_q_empty(kind), (q_seq[kind] & 1u) ^ 1u, ST_OS_WAIT_Q_EMPTY)) return false;
       if (lane == 0) {
         ptx::mbar_arrive_expect_tx(bar_q_full(kind), L::kTileBytes);
         for (int c = 0; c < copies; ++c)
@@ -216,7 +218,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       ++q_seq[kind];
       for (int t = g.t_lo; t < g.t_hi; ++t, ++ring_seq) {
         const uint32_t s = ring_seq % KR, ph = (ring_seq / KR) & 1u;
-        if (!WAIT(bar_ring_empty(s), ph ^ 1u, ST_OS_WAIT_RING_EMPTY)) return false;
+        if (!WAIT_BEHIND_PEERS(bar_ring_empty(s), ph ^ 1u, ST_OS_WAIT_RING_EMPTY)) return false;
         const bool left_out = blockIdx.x == 0 && (int)ring_seq == p.skip_ring_load;  // self-test of the bounded waits
         if (lane == 0 && !left_out) {
           ptx::mbar_arrive_expect_tx(bar_ring_full(s), L::kTileBytes);
@@ -239,7 +241,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       else
         dealer.deal(r.item[0], r.item[1]);
       const uint32_t i = n % kOsRecords;
-      if (!WAIT(bar_rec_empty(i), ((n / kOsRecords) & 1u) ^ 1u, ST_OS_WAIT_RECORD_EMPTY)) return false;
+      if (!WAIT_BEHIND_PEERS(bar_rec_empty(i), ((n / kOsRecords) & 1u) ^ 1u, ST_OS_WAIT_RECORD_EMPTY)) return false;
       if (lane == 0) {
         records[2 * i] = r.item[0];
         records[2 * i + 1] = r.item[1];
@@ -291,7 +293,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           ok = WAIT(bar_ring_full(s), ph, ST_OS_WAIT_RING_FULL);
           if (!ok) break;
           const uint32_t buf = ring_seq % kKsBuffers;
-          ok = WAIT(bar_tm_empty(buf), ((ring_seq / kKsBuffers) & 1u) ^ 1u, ST_OS_WAIT_TMEM_EMPTY);
+          ok = WAIT_BEHIND_PEERS(bar_tm_empty(buf), ((ring_seq / kKsBuffers) & 1u) ^ 1u, ST_OS_WAIT_TMEM_EMPTY);
           if (!ok) break;
           ptx::tc_fence_after_sync();
           if (ptx::elect_one()) {
@@ -357,7 +359,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                   ok = false;
                   break;
                 }
-                if (clock64() - t0 > p.wait_limit) {
+                if (clock64() - t0 > 2 * p.wait_limit) {
                   *abort_flag = 1;
                   report_status(p, ST_OS_WAIT_HEAD, g.bh);
                   ok = false;
@@ -391,7 +393,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           }
         }
         const uint32_t lb = (n_cols - 1) % kOsLseBuffers, lph = ((n_cols - 1) / kOsLseBuffers) & 1u;
-        ok = WAIT(bar_lse_empty(lb), lph ^ 1u, ST_OS_WAIT_LSE_EMPTY);
+        ok = WAIT_BEHIND_PEERS(bar_lse_empty(lb), lph ^ 1u, ST_OS_WAIT_LSE_EMPTY);
         if (!ok) break;
         lse_all[lb * kTile + i] = i < p.M ? -(mx + log2f(l)) : 0.f;
         __syncwarp();
@@ -399,7 +401,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       if (segment(r, 0, g) && (int)(n_rows++ % copies) == team) {
         const uint32_t pb = (n_rows - 1) % kOsPartBuffers, pph = ((n_rows - 1) / kOsPartBuffers) & 1u;
-        ok = WAIT(bar_part_full(pb), pph, ST_OS_WAIT_PART_FULL);
+        ok = WAIT_BEHIND_PEERS(bar_part_full(pb), pph, ST_OS_WAIT_PART_FULL);
         if (!ok) break;
         // the four warpgroups' states of this chunk, in the order of their tiles
         const float2* cell = part_s + pb * (kKsBuffers * kTile) + i;
@@ -481,7 +483,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           if (!ok) break;
           const uint32_t pb = n_rows % kOsPartBuffers, pph = (n_rows / kOsPartBuffers) & 1u;
           ++n_rows;
-          ok = WAIT(bar_part_empty(pb), pph ^ 1u, ST_OS_WAIT_PART_EMPTY);
+          ok = WAIT_BEHIND_PEERS(bar_part_empty(pb), pph ^ 1u, ST_OS_WAIT_PART_EMPTY);
           if (!ok) break;
           // a warpgroup without a tile in this chunk leaves (-inf, 0), which the merge skips
           if (live) part_s[(pb * kKsBuffers + j0) * kTile + tid_wg] = make_float2(m_run, l_run);
@@ -490,7 +492,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         } else {
           const uint32_t lb = n_cols % kOsLseBuffers, lph = (n_cols / kOsLseBuffers) & 1u;
           ++n_cols;
-          ok = WAIT(bar_lse_full(lb), lph, ST_OS_WAIT_LSE_FULL);
+          ok = WAIT_BEHIND_PEERS(bar_lse_full(lb), lph, ST_OS_WAIT_LSE_FULL);
           if (!ok) break;
           const float* lse_s = lse_all + lb * kTile;
           const int n_fold = p.fold_cols / kChunkCols;  // only the chunks that hold a query

@@ -170,7 +170,9 @@ size_t fcr_workspace_bytes(const fcr_problem* problem, int32_t num_sms);
  * Replaces `_flash_colreduce` (flash_colreduce/flash.py:277-308) together
  * with the tail of `flash_colreduce` (flash.py:377-385).
  *
- * Every wait inside the kernels is bounded (about one second).  A kernel whose
+ * Every wait inside the kernels is bounded (about one second; two or three for
+ * waits on warps or blocks that themselves wait, so that the one at the root
+ * reports first).  A kernel whose
  * wait expires gives up, leaves `out` unspecified and records a status code in
  * the workspace and in a per-device mailbox in mapped host memory; the NEXT
  * call of fcr_colreduce / fcr_colreduce_static on that device (or
@@ -319,8 +321,9 @@ int64_t fcr_launch_count(void);
 
 /*
  * Self-test of the bounded waits, for the calling thread's later
- * fcr_colreduce calls: `wait_limit_cycles` > 0 replaces the one-second bound
- * of every device-side wait (in SM clock cycles), and `skip_ring_load` >= 0
+ * fcr_colreduce calls: `wait_limit_cycles` > 0 replaces the one second from
+ * which the bound of every device-side wait is made (once to three times it, in
+ * SM clock cycles), and `skip_ring_load` >= 0
  * makes the first CTA of each kernel that streams tiles leave out its
  * skip_ring_load-th streamed-tile load, so that the waits on that tile expire: the kernels then
  * give up in an orderly way (no trap, no fault; tensor memory is released) and

@@ -126,7 +126,7 @@ DECODE = [(4, 24, 8192, 128), (64, 24, 8192, 256), (64, 24, 8192, 128), (40, 150
 @pytest.mark.parametrize("skip", [0, 3])
 def test_expired_wait_in_the_decode_kernels(no_debug_sync, m, heads, n, d, skip):
     """The CTA whose load is missing gives up, and so do the CTAs that wait for its chunk states; the call returns, reports
-    itself once, and the next call is right."""
+    the wait at the root once (the tile, or its product, in the CTA without it), and the next call is right."""
     from flash_colreduce_b200 import _native as nat
     from flash_colreduce_b200 import flash_colreduce
 
@@ -145,7 +145,9 @@ def test_expired_wait_in_the_decode_kernels(no_debug_sync, m, heads, n, d, skip)
     torch.cuda.synchronize()
     code = C.c_int32(-1)
     assert nat.lib.fcr_poll_device_status(C.byref(code)) == nat.FCR_ERR_DEVICE_TIMEOUT
-    assert 50 < code.value < 80 and "bounded wait" in nat.last_error()
+    # wait on the tile, or on its product: of the key-streaming kernels, of the one-sweep kernel
+    assert code.value in ((54, 57) if m <= 16 or d > 128 else (64, 67)), nat.last_error()
+    assert "block 0" in nat.last_error() and "bounded wait" in nat.last_error()
     assert nat.lib.fcr_poll_device_status(C.byref(code)) == nat.FCR_OK
     after = flash_colreduce(qd, kd, "sum", is_causal=True)
     assert torch.equal(before, after)
