@@ -148,8 +148,31 @@ def test_many_short_rows_inside_a_cuda_graph(monkeypatch):
                                       (400, 2047, 300), (400, 2048, 1), (400, 2049, 2049)])
 def test_rows_at_the_edge_of_one_sweep_step(dtype, rows, n, k):
     """A slice of one sweep step (8192 elements, 2048 for the small blocks) is kept in registers, one more element is
-    not; the values are made from the keys, so negative scores, both zeros and infinities come back bit for bit."""
+    not."""
     g = torch.Generator().manual_seed(n + k)
     s = torch.randn(rows, n, generator=g).to(dtype)
     s[0, : min(4, n)] = torch.tensor([float("inf"), float("-inf"), 0.5, -0.5][: min(4, n)]).to(dtype)
     _check(s, k)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows,n,k", [(3, 8192, 8192), (3, 8193, 8193), (400, 2048, 2048), (3, 8192, 5000), (2, 16384, 9000)])
+def test_values_come_back_bit_for_bit(dtype, rows, n, k):
+    """The values are made from the ordering keys: negative scores, both zeros, subnormals, infinities and NaNs of either
+    sign with their payloads are the bits that went in (compared as integers; the first cases select every element)."""
+    from flash_colreduce_b200 import topk_columns
+
+    bits = torch.int32 if dtype == torch.float32 else torch.int16
+    special = {torch.float32: [0x00000000, 0x80000000, 0x7F800000, 0xFF800000, 0x7FC01234, 0xFFC05678, 0x00000001, 0x80000001],
+               torch.float16: [0x0000, 0x8000, 0x7C00, 0xFC00, 0x7E12, 0xFE34, 0x0001, 0x8001],
+               torch.bfloat16: [0x0000, 0x8000, 0x7F80, 0xFF80, 0x7FC5, 0xFFD6, 0x0001, 0x8001]}[dtype]
+    g = torch.Generator().manual_seed(n)
+    s = torch.randn(rows, n, generator=g).to(dtype).view(bits).clone()
+    width = 1 << (32 if bits == torch.int32 else 16)
+    s[:, 3:3 + 8 * 7:7] = torch.tensor([x - width if x >= width // 2 else x for x in special], dtype=bits)
+    vals, idx = topk_columns(s.view(dtype).to(_dev()), k)
+    idx = idx.cpu()
+    assert (idx[:, 1:] > idx[:, :-1]).all() and int(idx.min()) >= 0 and int(idx.max()) < n
+    assert torch.equal(vals.cpu().view(bits), torch.gather(s, 1, idx))
+    if k == n:
+        assert torch.equal(vals.cpu().view(bits), s)
