@@ -44,7 +44,7 @@ def _tma_ready(x: torch.Tensor) -> torch.Tensor:
     for dim in range(3):
         if x.shape[dim] > 1 and (x.stride(dim) <= 0 or x.stride(dim) % unit != 0):
             ok = False
-    return x if ok else x.contiguous()
+    return x if ok else x.clone(memory_format=torch.contiguous_format)  # (contiguous() keeps an unaligned base)
 
 
 # What a call signature (shapes, strides, types, devices, options; no data, no addresses) comes to: whether each

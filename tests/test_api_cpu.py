@@ -54,3 +54,25 @@ def test_signature_is_the_reference_operator_signature():
     assert all(p.kind is inspect.Parameter.POSITIONAL_OR_KEYWORD for p in params.values())
     naive = inspect.signature(fc.naive_colreduce).parameters
     assert list(naive)[:5] == ["query", "key", "reduction", "is_causal", "scale"]  # naive.py:8-14
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_operands_tma_cannot_describe_are_copied(dtype):
+    """An unaligned base, a transposed inner dimension, rows of odd width, a head dimension that is no multiple of 16 bytes:
+    what goes in has the values, unit inner stride, strides of whole 16 bytes and an aligned base."""
+    from flash_colreduce_b200.op import _tma_ready
+
+    unit = 16 // torch.empty(0, dtype=dtype).element_size()
+    x = torch.randn(2, 3, 5, 16).to(dtype)
+    shifted = torch.empty(x.numel() + 1, dtype=dtype)[1:].view_as(x).copy_(x)
+    assert shifted.is_contiguous() and shifted.data_ptr() % 16 != 0
+    inner = x.transpose(2, 3).contiguous().transpose(2, 3)
+    wide = torch.zeros(2, 3, 5, 17, dtype=dtype)[..., :16].copy_(x)
+    for y in (shifted, inner, wide, x[..., :13]):
+        z = _tma_ready(y)
+        assert torch.equal(z[..., :y.shape[-1]], y) and not z[..., y.shape[-1]:].any()
+        assert z.data_ptr() % 16 == 0 and z.stride(3) == 1 and z.shape[-1] % unit == 0
+        assert all(z.stride(i) % unit == 0 for i in range(3))
+    assert _tma_ready(x) is x
+    bmhd = torch.randn(2, 5, 3, 16).to(dtype).transpose(1, 2)
+    assert _tma_ready(bmhd) is bmhd
