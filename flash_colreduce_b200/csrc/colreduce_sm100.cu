@@ -1160,14 +1160,20 @@ static int launch_onesweep_d(int d_pad, const CUtensorMap& map_q, const CUtensor
   return launch_onesweep<128, RED>(map_q, map_k, pp, chunk_state, counters, idesc_cols, copies, ctas, stream);
 }
 
+// A plan and what a call needs beside it.
+struct CallPlan {
+  fcr_plan plan;
+  int chunks;  // per head, of the one-sweep kernel (0: the plan does not take it)
+};
+
 // Bytes a plan cannot do without: the score cache and the one-sweep kernel's scratch are each the last
 // region of the workspace and optional (without them the columns pass sweeps K a second time).
-static int64_t min_workspace_bytes(const fcr_problem& pr, const fcr_plan& pl, int sms) {
-  return pl.score_cache ? pl.off_scores : pl.workspace_bytes - onesweep_bytes(pr, pl, sms);
+static int64_t min_workspace_bytes(const fcr_problem& pr, const CallPlan& cp) {
+  return cp.plan.score_cache ? cp.plan.off_scores : cp.plan.workspace_bytes - onesweep_bytes(pr, cp.plan, cp.chunks);
 }
 
-static int check_workspace(const fcr_problem& pr, const fcr_plan& pl, int sms, const void* ws, size_t ws_bytes) {
-  const int64_t needed = min_workspace_bytes(pr, pl, sms);
+static int check_workspace(const fcr_problem& pr, const CallPlan& cp, const void* ws, size_t ws_bytes) {
+  const int64_t needed = min_workspace_bytes(pr, cp);
   if (!ws) return fail(FCR_ERR_WORKSPACE, "workspace is null");
   if ((reinterpret_cast<uintptr_t>(ws) & 255u) != 0)
     return fail(FCR_ERR_WORKSPACE, "workspace must be 256-byte aligned");
@@ -1355,7 +1361,7 @@ size_t fcr_workspace_bytes(const fcr_problem* problem, int32_t num_sms) {
 struct PlanCacheEntry {
   fcr_problem problem;
   int device;
-  fcr_plan plan;
+  CallPlan plan;
 };
 static bool same_problem(const fcr_problem& a, const fcr_problem& b) {
   return a.B == b.B && a.H == b.H && a.M == b.M && a.N == b.N && a.D == b.D &&
@@ -1365,7 +1371,7 @@ static bool same_problem(const fcr_problem& a, const fcr_problem& b) {
          memcmp(&a.scale, &b.scale, sizeof(float)) == 0 && a.causal_offset == b.causal_offset &&
          a.mean_M == b.mean_M && a.mean_N == b.mean_N;
 }
-static int plan_for_call(const fcr_problem& pr, const DeviceInfo& dev, const fcr_plan** out) {
+static int plan_for_call(const fcr_problem& pr, const DeviceInfo& dev, const CallPlan** out) {
   constexpr int kEntries = 8;
   static thread_local PlanCacheEntry cache[kEntries];
   static thread_local int used = 0, next = 0;
@@ -1375,9 +1381,10 @@ static int plan_for_call(const fcr_problem& pr, const DeviceInfo& dev, const fcr
       return FCR_OK;
     }
   std::string err;
-  fcr_plan pl;
-  const int rc = plan_problem(pr, dev.sms, pl, err);
+  CallPlan pl;
+  const int rc = plan_problem(pr, dev.sms, pl.plan, err);
   if (rc != FCR_OK) return fail(rc, err);
+  pl.chunks = onesweep_chunks(pr, pl.plan, dev.sms);
   PlanCacheEntry& e = cache[next];
   e.problem = pr;
   e.device = dev.index;
@@ -1389,11 +1396,12 @@ static int plan_for_call(const fcr_problem& pr, const DeviceInfo& dev, const fcr
 }
 
 // The operator proper, behind fcr_colreduce and fcr_colreduce_static.
-static int run_colreduce(const fcr_problem& pr, const fcr_plan& pl, const DeviceInfo& dev, const void* q,
+static int run_colreduce(const fcr_problem& pr, const CallPlan& cp, const DeviceInfo& dev, const void* q,
                          const void* k, void* out, int32_t out_dtype, void* workspace,
                          size_t workspace_bytes, cudaStream_t stream) {
-  int rc = check_workspace(pr, pl, dev.sms, workspace, workspace_bytes);
+  int rc = check_workspace(pr, cp, workspace, workspace_bytes);
   if (rc != FCR_OK) return rc;
+  const fcr_plan& pl = cp.plan;
   uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
   t_device = dev.index;
   int* const mailbox = dev.mailbox_dev;
@@ -1425,15 +1433,14 @@ static int run_colreduce(const fcr_problem& pr, const fcr_plan& pl, const Device
     };
     fill(false);
     // One sweep over K instead of two, when the workspace has room for the chunk states.
-    const int chunks = onesweep_chunks(pr, pl, dev.sms);
-    if (chunks > 0 && (int64_t)workspace_bytes >= pl.workspace_bytes) {
+    if (cp.chunks > 0 && (int64_t)workspace_bytes >= pl.workspace_bytes) {
       fill_mean(pp, pr.reduction, pr.is_causal, pr.mean_M > 0 ? pr.mean_M : pr.M,
                 pr.mean_N > 0 ? pr.mean_N : pr.N);
       pp.out = out;
       pp.out_dtype = out_dtype;
-      pp.n_split = chunks;
-      pp.n_items = pp.BH * chunks;
-      uint8_t* region = ws + (pl.workspace_bytes - onesweep_bytes(pr, pl, dev.sms));
+      pp.n_split = cp.chunks;
+      pp.n_items = pp.BH * cp.chunks;
+      uint8_t* region = ws + (pl.workspace_bytes - onesweep_bytes(pr, pl, cp.chunks));
       int* counters = reinterpret_cast<int*>(region);
       float2* chunk_state = reinterpret_cast<float2*>(region + onesweep_counter_bytes(pr));
       e = cudaMemsetAsync(counters, 0, onesweep_counter_bytes(pr), stream);
@@ -1553,7 +1560,7 @@ int fcr_colreduce(const fcr_problem* problem, const void* q, const void* k, void
   if (rc != FCR_OK) return rc;
   rc = check_mailbox(*dev, nullptr);  // a wait that expired in an earlier call is reported here
   if (rc != FCR_OK) return rc;
-  const fcr_plan* pl = nullptr;
+  const CallPlan* pl = nullptr;
   rc = plan_for_call(*problem, *dev, &pl);
   if (rc != FCR_OK) return rc;
   return run_colreduce(*problem, *pl, *dev, q, k, out, out_dtype, workspace, workspace_bytes,
@@ -1690,10 +1697,10 @@ int fcr_colreduce_static(const fcr_problem* problem, const void* q, const void* 
   if (rc != FCR_OK) return rc;
   rc = check_mailbox(*dev, nullptr);
   if (rc != FCR_OK) return rc;
-  const fcr_plan* pl = nullptr;
+  const CallPlan* pl = nullptr;
   rc = plan_for_call(*problem, *dev, &pl);
   if (rc != FCR_OK) return rc;
-  const int64_t needed = min_workspace_bytes(*problem, *pl, dev->sms);
+  const int64_t needed = min_workspace_bytes(*problem, *pl);
   if ((size_t)needed > kStaticScratchBytes)
     return fail(FCR_ERR_WORKSPACE,
                 "this problem needs " + std::to_string(needed) +

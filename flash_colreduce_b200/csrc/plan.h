@@ -238,9 +238,8 @@ inline int onesweep_copies(int M) { return M <= 32 ? 4 : (M <= 64 ? 2 : 1); }
 inline int64_t onesweep_counter_bytes(const fcr_problem& p) {
   return align_up64(((int64_t)p.B * p.H * 4 + 1) * 4, 256);
 }
-inline int64_t onesweep_bytes(const fcr_problem& p, const fcr_plan& pl, int num_sms) {
-  const int64_t s = onesweep_chunks(p, pl, num_sms);
-  return s == 0 ? 0 : onesweep_counter_bytes(p) + align_up64(s * p.B * p.H * pl.m_pad * 8, 256);
+inline int64_t onesweep_bytes(const fcr_problem& p, const fcr_plan& pl, int chunks) {
+  return chunks == 0 ? 0 : onesweep_counter_bytes(p) + align_up64((int64_t)chunks * p.B * p.H * pl.m_pad * 8, 256);
 }
 
 inline int plan_problem(const fcr_problem& p, int num_sms, fcr_plan& pl, std::string& err) {
@@ -416,7 +415,7 @@ inline int plan_problem(const fcr_problem& p, int num_sms, fcr_plan& pl, std::st
     pl.off_scores = o;
     o += align_up64(score_bytes, 256);
   }
-  o += onesweep_bytes(p, pl, num_sms);
+  o += onesweep_bytes(p, pl, onesweep_chunks(p, pl, num_sms));
   pl.workspace_bytes = o;
   return FCR_OK;
 }

@@ -257,7 +257,7 @@ int fcr_colreduce_sharded(const fcr_problem* local, const fcr_shard* shard, int3
     const size_t elem = lp.in_dtype == FCR_F32 ? 4 : 2;
     for (int r = 0; r < shard->n_ranges; ++r) {
       const fcr_problem sp = slice_problem(lp, shard->row_lo[r], shard->row_hi[r]);
-      const fcr_plan* pl = nullptr;
+      const CallPlan* pl = nullptr;
       rc = plan_for_call(sp, *dev, &pl);
       if (rc != FCR_OK) return rc;
       const uint8_t* q_rows = reinterpret_cast<const uint8_t*>(q) + (size_t)shard->row_lo[r] * lp.q_strides[2] * elem;

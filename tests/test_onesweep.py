@@ -24,7 +24,7 @@ extern "C" int chunks_of(int B, int H, int M, int N, int D, int causal, int dtyp
   std::string err;
   if (fcr::plan_problem(p, sms, pl, err) != FCR_OK) return -1;
   out[0] = pl.key_stream; out[1] = pl.score_cache; out[2] = pl.d_pad; out[3] = pl.n_pad / 128; out[4] = pl.m_pad;
-  out[5] = pl.workspace_bytes; out[6] = fcr::onesweep_bytes(p, pl, sms); out[7] = fcr::onesweep_counter_bytes(p);
+  out[5] = pl.workspace_bytes; out[6] = fcr::onesweep_bytes(p, pl, fcr::onesweep_chunks(p, pl, sms)); out[7] = fcr::onesweep_counter_bytes(p);
   out[8] = pl.off_part_l + 4ll * pl.row_splits * B * H * pl.m_pad;
   return fcr::onesweep_chunks(p, pl, sms);
 }
@@ -236,6 +236,14 @@ def test_the_exchange_orders_the_memory_of_all_lanes():
     publish = code[code.index("__stcg("):code.index("red_release_add(")]
     collect = code[code.rindex("ld_acquire("):code.index("__ldcg(")]
     assert "__syncwarp()" in publish and "__syncwarp()" in collect
+
+
+def test_the_chunks_are_chosen_with_the_plan():
+    """A repeated problem plans nothing: the search for the chunk count runs where a plan is made, not in every call."""
+    with open(os.path.join(ROOT, "flash_colreduce_b200", "csrc", "colreduce_sm100.cu")) as f:
+        code = re.sub(r"//[^\n]*", "", f.read())
+    planner, rest = code.split("static int plan_for_call(", 1)[1].split("\n}\n", 1)
+    assert planner.count("onesweep_chunks(") == 1 and code.count("onesweep_chunks(") == 1
 
 
 def test_which_shapes_take_it_and_where_its_scratch_lies(planner):
