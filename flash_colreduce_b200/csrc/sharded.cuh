@@ -139,8 +139,9 @@ static fcr_problem slice_problem(const fcr_problem& local, int lo, int hi) {
   return p;
 }
 
-static int sharded_layout(const fcr_problem& local, const fcr_shard& sh, const DeviceInfo& dev, int64_t* off_part,
-                          int64_t* total) {
+// Without `one_sweep` the layout leaves out that kernel's scratch, as fcr_colreduce lets its caller do.
+static int sharded_layout(const fcr_problem& local, const fcr_shard& sh, const DeviceInfo& dev, bool one_sweep,
+                          int64_t* off_part, int64_t* total) {
   int64_t need = 0;
   for (int r = 0; r < sh.n_ranges; ++r) {
     const fcr_problem p = slice_problem(local, sh.row_lo[r], sh.row_hi[r]);
@@ -148,7 +149,8 @@ static int sharded_layout(const fcr_problem& local, const fcr_shard& sh, const D
     fcr_plan pl;
     const int rc = plan_problem(p, dev.sms, pl, err);
     if (rc != FCR_OK) return fail(rc, err);
-    need = std::max<int64_t>(need, pl.workspace_bytes);
+    const int64_t scratch = one_sweep ? 0 : onesweep_bytes(p, pl, onesweep_chunks(p, pl, dev.sms));
+    need = std::max<int64_t>(need, pl.workspace_bytes - scratch);
   }
   need = align_up64(need, 256);
   *off_part = need;
@@ -217,7 +219,7 @@ size_t fcr_sharded_workspace_bytes(const fcr_problem* local, const fcr_shard* sh
   const DeviceInfo* dev = nullptr;
   if (device_info(&dev, false) != FCR_OK) return 0;
   int64_t off_part = 0, total = 0;
-  if (sharded_layout(*local, *shard, *dev, &off_part, &total) != FCR_OK) return 0;
+  if (sharded_layout(*local, *shard, *dev, true, &off_part, &total) != FCR_OK) return 0;
   return (size_t)total;
 }
 
@@ -247,10 +249,11 @@ int fcr_colreduce_sharded(const fcr_problem* local, const fcr_shard* shard, int3
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(acc)");
   if (heads > 0) {
     int64_t off_part = 0, total = 0;
-    rc = sharded_layout(lp, *shard, *dev, &off_part, &total);
+    rc = sharded_layout(lp, *shard, *dev, true, &off_part, &total);
+    if (rc == FCR_OK && (int64_t)workspace_bytes < total) rc = sharded_layout(lp, *shard, *dev, false, &off_part, &total);
     if (rc != FCR_OK) return rc;
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0 || (int64_t)workspace_bytes < total)
-      return fail(FCR_ERR_WORKSPACE, "workspace missing, misaligned or smaller than fcr_sharded_workspace_bytes() = " +
+      return fail(FCR_ERR_WORKSPACE, "workspace missing, misaligned or smaller than the required " +
                                          std::to_string(total));
     uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
     float* part = reinterpret_cast<float*>(ws + off_part);

@@ -284,7 +284,8 @@ int fcr_comm_destroy(void* comm);
  * scale.  acc: device fp32 (total_heads, N), scratch for the partial vectors;
  * out: device (total_heads, N) of out_dtype, the full result on every rank.
  * workspace: at least fcr_sharded_workspace_bytes(local, shard), 256-byte
- * aligned.  comm may be NULL when shard->world == 1.  Everything is queued on
+ * aligned (the scratch of the one-sweep decode kernel is optional as for
+ * fcr_colreduce: an array smaller by it is accepted).  comm may be NULL when shard->world == 1.  Everything is queued on
  * `stream`: a memset of acc, fcr_colreduce's kernels per row range, one small
  * fold kernel per range, ncclAllReduce, the finalize kernel; no host
  * synchronisation.

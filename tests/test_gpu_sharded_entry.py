@@ -67,3 +67,39 @@ def test_row_ranges_of_a_multi_rank_plan_add_up(world, m, n, causal, reduction):
         total = torch.maximum(total, part) if reduction == "max" else total + part
     assert rows_seen == m
     assert_parity(total[None], oracle_colreduce(q, k, reduction, causal), reduction)
+
+
+def test_the_one_sweep_scratch_is_optional():
+    """A decode shape's workspace without the chunk states is accepted, as by fcr_colreduce, and runs two sweeps."""
+    from flash_colreduce_b200 import _native as nat
+
+    dev, heads, m, n = _dev(), 3, 64, 3000
+    g = torch.Generator().manual_seed(7)
+    q = torch.randn(1, heads, m, 64, generator=g).half()
+    k = torch.randn(1, heads, n, 64, generator=g).half()
+    qd, kd = q.to(dev), k.to(dev)
+    prob = nat.make_problem(1, heads, m, n, 64, qd.stride(), kd.stride(), nat.FCR_F16, nat.FCR_SUM, True, 1 / math.sqrt(64))
+    sh = nat.Shard()
+    nat.check(nat.lib.fcr_plan_shards(heads, m, 1, 0, C.byref(sh)), "fcr_plan_shards")
+    pl = nat.plan(prob, 0)
+    states = int(pl.off_part_l) + 4 * int(pl.row_splits) * heads * int(pl.m_pad)
+    least = (states + 255) // 256 * 256 + (heads * n * 4 + 255) // 256 * 256
+    full = nat.lib.fcr_sharded_workspace_bytes(C.byref(prob), C.byref(sh))
+    assert least < full
+    acc = torch.empty(heads, n, dtype=torch.float32, device=dev)
+
+    def run(size):
+        ws = torch.empty(size, dtype=torch.uint8, device=dev)
+        out = torch.empty(heads, n, dtype=torch.float32, device=dev)
+        before = nat.lib.fcr_launch_count()
+        rc = nat.lib.fcr_colreduce_sharded(C.byref(prob), C.byref(sh), heads, qd.data_ptr(), kd.data_ptr(), acc.data_ptr(),
+                                           out.data_ptr(), nat.FCR_F32, ws.data_ptr(), size, None,
+                                           torch.cuda.current_stream().cuda_stream)
+        return rc, out, nat.lib.fcr_launch_count() - before
+
+    want = oracle_colreduce(q, k, "sum", True)
+    for size, kernels in ((full, 3), (full - 256, 5), (least, 5)):  # the operator's one or three, the fold, the cast
+        rc, out, launches = run(size)
+        assert rc == nat.FCR_OK and launches == kernels, nat.last_error()
+        assert_parity(out[None], want, "sum")
+    assert run(least - 256)[0] == nat.FCR_ERR_WORKSPACE
