@@ -43,7 +43,7 @@ constexpr int kOsLseBuffers = 4;    // chunks whose lse values may wait for thei
 constexpr int kOsPartBuffers = 4;
 // Records announced to the other warps.  The TMA warp deals one ahead; the statistics warps may lag by the part buffers.
 constexpr int kOsRecords = 16;
-constexpr int kOsEnd = -2;  // the rows item of the last record
+constexpr int kOsEnd = -2;  // in the place of a head: the last record
 constexpr int kOsChunk = 32;  // accumulator columns per tensor-memory load (736 threads: 80 registers)
 
 // A missing tile shows first in its own CTA (bound 1: Q_FULL, RING_FULL, TMEM_FULL, DRAIN), then in the CTAs that wait for
@@ -78,8 +78,9 @@ struct OneSweepSmem {
   static constexpr int off_bars = off_lse + kOsLseBuffers * kTile * 4;
   static constexpr int kNumBars = 4 + 2 * KR + 2 * kKsBuffers + 2 * kOsPartBuffers + 2 * kOsLseBuffers + 2 * kOsRecords;
   static constexpr int off_misc = off_bars + 8 * kNumBars;
-  static constexpr int off_records = off_misc + 16;              // int [kOsRecords][2]: rows item, columns item
-  static constexpr int off_held = off_records + 8 * kOsRecords;  // int [kOneSweepHeld], the dealer's
+  static constexpr int off_records = off_misc + 16;               // int4 [kOsRecords][2]: rows pass, columns pass (head, chunk, tiles)
+  static constexpr int off_held = off_records + 32 * kOsRecords;  // int [kOneSweepHeld], the dealer's
+  static_assert(off_records % 16 == 0, "records are read as 16 bytes");
   static constexpr int kDynamicBytes = off_held + 4 * kOneSweepHeld;
   static_assert(kDynamicBytes <= 232448, "exceeds the 227 KB shared memory of an sm_100 CTA");
 };
@@ -119,7 +120,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::off_misc + 4);
   float2* const part_s = reinterpret_cast<float2*>(smem + L::off_part);
   float* const lse_all = reinterpret_cast<float*>(smem + L::off_lse);
-  volatile int* const records = reinterpret_cast<volatile int*>(smem + L::off_records);
+  int4* const records = reinterpret_cast<int4*>(smem + L::off_records);
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // warp-uniform for the compiler
   const int lane = (int)(threadIdx.x & 31);
@@ -173,26 +174,26 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   if (threadIdx.x == 0) ptx::grid_launch_dependents();
   if (p.clear_status && blockIdx.x == 0 && threadIdx.x < 4) p.status[threadIdx.x] = 0;
 
-  // A record is the rows pass of one chunk (kind 0) and then the columns pass of another (kind 1), or one of them.
+  // A record is the rows pass of one chunk (kind 0) and then the columns pass of another (kind 1), or one of them.  The
+  // TMA warp decodes it once (two 64-bit divisions a chunk); the others read it where they need it and give it back.
   const int S = p.n_split;
-  struct Record { int item[2]; };
   struct Segment { int bh, sp, t_lo, t_hi; };
-  auto segment = [&](const Record& r, int kind, Segment& g) {
-    const int item = kind == 0 ? r.item[0] : r.item[1];
-    if (item < 0) return false;
-    keystream_item(S, p.key_tiles, item, g.bh, g.sp, g.t_lo, g.t_hi);
-    return true;
+  // Waits for the n-th record; false at the end, or when the wait expired (then not ok).
+  auto next_record = [&](uint32_t n, bool& ok) {
+    ok = WAIT_BEHIND_PEERS(bar_rec_full(n % kOsRecords), (n / kOsRecords) & 1u, ST_OS_WAIT_RECORD_FULL);
+    return ok && __shfl_sync(0xffffffffu, records[2 * (n % kOsRecords)].x, 0) != kOsEnd;
   };
-  // The n-th record, as the TMA warp announced it; false at the end, or when the wait for it expired (then not ok).
-  auto next_record = [&](uint32_t n, Record& r, bool& ok) {
-    const uint32_t i = n % kOsRecords;
-    ok = WAIT_BEHIND_PEERS(bar_rec_full(i), (n / kOsRecords) & 1u, ST_OS_WAIT_RECORD_FULL);
-    if (!ok) return false;
-    r.item[0] = records[2 * i];
-    r.item[1] = records[2 * i + 1];
+  auto segment = [&](uint32_t n, int kind, Segment& g) {
+    const int4 v = records[2 * (n % kOsRecords) + kind];  // (shuffled: warp-uniform for the compiler)
+    g.bh = __shfl_sync(0xffffffffu, v.x, 0);
+    g.sp = __shfl_sync(0xffffffffu, v.y, 0);
+    g.t_lo = __shfl_sync(0xffffffffu, v.z, 0);
+    g.t_hi = __shfl_sync(0xffffffffu, v.w, 0);
+    return g.bh >= 0;
+  };
+  auto record_done = [&](uint32_t n) {
     __syncwarp();
-    if (lane == 0) ptx::mbar_arrive(bar_rec_empty(i));
-    return r.item[0] != kOsEnd;
+    if (lane == 0) ptx::mbar_arrive(bar_rec_empty(n % kOsRecords));
   };
 
   if (warp == kKsProducerWarp) {
@@ -202,8 +203,12 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const uint64_t keep = ptx::l2_policy_evict_normal(), drop = ptx::l2_policy_evict_first();
     uint32_t ring_seq = 0, q_seq[2] = {0, 0};
     bool ok = true;
+    // self-test of the bounded waits: this load is left out
+    const uint32_t skip_seq = blockIdx.x == 0 ? (uint32_t)p.skip_ring_load : ~0u;
+    int ticket = 0;  // lane 0: the next ticket, on its way
     // one pass over a chunk: its head's query tile (a head's chunks go to different CTAs), then its key tiles
-    auto load_segment = [&](const Segment& g, int kind) {
+    auto load_segment = [&](const Segment& g, int kind, bool draw) {
+      const int draw_at = draw ? max(g.t_lo, g.t_hi - 2) : -1;
       const int b = g.bh / p.H, h = g.bh - b * p.H;
       if (!WAIT_BEHIND_PEERS(bar_q_empty(kind), (q_seq[kind] & 1u) ^ 1u, ST_OS_WAIT_Q_EMPTY)) return false;
       if (lane == 0) {
@@ -219,8 +224,8 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       for (int t = g.t_lo; t < g.t_hi; ++t, ++ring_seq) {
         const uint32_t s = ring_seq % KR, ph = (ring_seq / KR) & 1u;
         if (!WAIT_BEHIND_PEERS(bar_ring_empty(s), ph ^ 1u, ST_OS_WAIT_RING_EMPTY)) return false;
-        const bool left_out = blockIdx.x == 0 && (int)ring_seq == p.skip_ring_load;  // self-test of the bounded waits
-        if (lane == 0 && !left_out) {
+        if (t == draw_at && lane == 0) ticket = atomicAdd(ticket_count, 1);
+        if (ring_seq != skip_seq && ptx::elect_one()) {
           ptx::mbar_arrive_expect_tx(bar_ring_full(s), L::kTileBytes);
 #pragma unroll
           for (int hf = 0; hf < L::kHalves; ++hf)
@@ -234,17 +239,21 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     uint32_t n = 0;  // records so far
     OneSweepDealer dealer;
     dealer.start(S, p.n_items, reinterpret_cast<int*>(smem + L::off_held), __shfl_sync(0xffffffffu, first_ticket, 0));
-    Record r;
+    Segment r[2];  // the record dealt last
     auto announce = [&]() {
-      if (dealer.finished())
-        r.item[0] = kOsEnd;
-      else
-        dealer.deal(r.item[0], r.item[1]);
+      int item[2] = {kOsEnd, -1};
+      if (!dealer.finished()) dealer.deal(item[0], item[1]);
+#pragma unroll
+      for (int kind = 0; kind < 2; ++kind) {
+        r[kind].bh = __shfl_sync(0xffffffffu, item[kind], 0);
+        if (r[kind].bh >= 0)
+          keystream_item(S, p.key_tiles, r[kind].bh, r[kind].bh, r[kind].sp, r[kind].t_lo, r[kind].t_hi);
+      }
       const uint32_t i = n % kOsRecords;
       if (!WAIT_BEHIND_PEERS(bar_rec_empty(i), ((n / kOsRecords) & 1u) ^ 1u, ST_OS_WAIT_RECORD_EMPTY)) return false;
       if (lane == 0) {
-        records[2 * i] = r.item[0];
-        records[2 * i + 1] = r.item[1];
+        records[2 * i] = make_int4(r[0].bh, r[0].sp, r[0].t_lo, r[0].t_hi);
+        records[2 * i + 1] = make_int4(r[1].bh, r[1].sp, r[1].t_lo, r[1].t_hi);
         ptx::mbar_arrive(bar_rec_full(i));
       }
       __syncwarp();
@@ -252,41 +261,36 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       return true;
     };
     ok = announce();
-    while (ok && r.item[0] != kOsEnd) {
+    while (ok && r[0].bh != kOsEnd) {
       const bool draw = dealer.needs_ticket(), first = n == 1;
-      // Asked for here, needed after the rows pass's loads.  The first one waits until a tile has landed: by then every
-      // CTA of the launch has had its turn, and a chunk that an idle SM could have does not queue up behind another.
-      int ticket = 0;
-      if (draw && !first && lane == 0) ticket = atomicAdd(ticket_count, 1);
-      Segment g;
-      if (segment(r, 0, g)) ok = load_segment(g, 0);
+      // Drawn with the requests of the rows pass's last tiles: not earlier, because a CTA that is a little ahead would
+      // take a chunk that another SM will be free for (8 heads, 64 x 32768, two chunks per CTA: 34.7 us when drawn a
+      // rows pass earlier, 26.7 here).  For the same reason a first chunk that about fits the ring draws once a tile
+      // has landed: by then every CTA of the launch has had its turn.
+      const bool rows = r[0].bh >= 0, small = first && rows && r[0].t_hi - r[0].t_lo <= KR + 1;
+      if (rows) ok = load_segment(r[0], 0, draw && !small);
+      if (ok && small && ring_seq <= KR) ok = WAIT(bar_ring_full(0), 0, ST_OS_WAIT_RING_FULL);  // (else a slot came back)
       if (!ok) break;
-      if (first) {
-        if (ring_seq <= KR) ok = WAIT(bar_ring_full(0), 0, ST_OS_WAIT_RING_FULL);  // (else a slot has been given back)
-        if (!ok) break;
-        if (draw && lane == 0) ticket = atomicAdd(ticket_count, 1);
-      }
-      const Record now = r;
+      if (draw && (small || !rows) && lane == 0) ticket = atomicAdd(ticket_count, 1);
+      const Segment cols = r[1];
       if (draw) dealer.draw(__shfl_sync(0xffffffffu, ticket, 0));
       ok = announce();
       if (!ok) break;
-      if (segment(now, 1, g)) ok = load_segment(g, 1);
+      if (cols.bh >= 0) ok = load_segment(cols, 1, false);
     }
   } else if (warp < kOsStatWarp && warp >= kKsMmaWarp) {
     // ------------------------------------------------------------ MMA warps
     const uint32_t my_turn = (uint32_t)(warp - kKsMmaWarp);
     uint32_t ring_seq = 0, q_seq[2] = {0, 0};
     bool ok = true;
-    Record r;
-    for (uint32_t n = 0; ok && next_record(n, r, ok); ++n) {
-#pragma unroll
+    for (uint32_t n = 0; ok && next_record(n, ok); ++n) {
+#pragma unroll 1
       for (int kind = 0; kind < 2; ++kind) {
         Segment g;
-        if (!ok || !segment(r, kind, g)) continue;
-        ok = WAIT(bar_q_full(kind), q_seq[kind] & 1u, ST_OS_WAIT_Q_FULL);
+        if (!ok || !segment(n, kind, g)) continue;
+        ok = WAIT(bar_q_full(kind), (kind == 0 ? q_seq[0]++ : q_seq[1]++) & 1u, ST_OS_WAIT_Q_FULL);
         if (!ok) continue;
         ptx::tc_fence_after_sync();
-        ++q_seq[kind];
         for (int t = g.t_lo; t < g.t_hi; ++t, ++ring_seq) {
           if (ring_seq % kOsMmaWarps != my_turn) continue;
           const uint32_t s = ring_seq % KR, ph = (ring_seq / KR) & 1u;
@@ -327,6 +331,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (ptx::elect_one()) ptx::umma_commit(bar_q_empty(kind));
         __syncwarp();
       }
+      if (ok) record_done(n);
     }
     // The last commits cover every MMA issued by either warp: no asynchronous arrive is outstanding when the CTA retires.
     if (ok && q_seq[0] > 0) ok = WAIT(bar_q_empty(0), (q_seq[0] - 1) & 1u, ST_OS_WAIT_DRAIN);
@@ -343,63 +348,70 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     // soon as the record before it is published, a whole rows pass before the columns pass needs the values.  (It waits
     // for chunks of smaller tickets only, never for the record's own rows.)
     uint32_t n_rows = 0, n_cols = 0;  // passes so far; the teams take them in turn
-    Record r;
-    for (uint32_t n = 0; ok && next_record(n, r, ok); ++n) {
+    // The head of this team's last columns pass: a CTA that holds several chunks of one head folds its states once
+    // (131 states took 9 us; 2 heads, 128 x 100000: 47 us without, 43 with) and copies the values of that pass.
+    int lse_head = -1;
+    for (uint32_t n = 0; ok && next_record(n, ok); ++n) {
       Segment g;
-      if (segment(r, 1, g) && (int)(n_cols++ % copies) == team) {
-        // every chunk of the head has been counted by this warp of whichever CTA folded it
-        if (lane == 0) {
-          const int* count = head_count + (size_t)g.bh * kOsStatWarps + w;
-          if (ptx::ld_acquire(count) < S) {
-            const long long t0 = clock64();
-            uint32_t spins = 0;
-            while (ptx::ld_acquire(count) < S) {
-              if ((++spins & 7u) == 0) {
-                if (*abort_flag) {
-                  ok = false;
-                  break;
-                }
-                if (clock64() - t0 > 2 * p.wait_limit) {
-                  *abort_flag = 1;
-                  report_status(p, ST_OS_WAIT_HEAD, g.bh);
-                  ok = false;
-                  break;
+      if (segment(n, 1, g) && (int)(n_cols++ % copies) == team) {
+        float neg_lse = lse_all[((n_cols - 1 - copies) % kOsLseBuffers) * kTile + i];
+        if (g.bh != lse_head) {
+          // every chunk of the head has been counted by this warp of whichever CTA folded it
+          if (lane == 0) {
+            const int* count = head_count + (size_t)g.bh * kOsStatWarps + w;
+            if (ptx::ld_acquire(count) < S) {
+              const long long t0 = clock64();
+              uint32_t spins = 0;
+              while (ptx::ld_acquire(count) < S) {
+                if ((++spins & 7u) == 0) {
+                  if (*abort_flag) {
+                    ok = false;
+                    break;
+                  }
+                  if (clock64() - t0 > 2 * p.wait_limit) {
+                    *abort_flag = 1;
+                    report_status(p, ST_OS_WAIT_HEAD, g.bh);
+                    ok = false;
+                    break;
+                  }
                 }
               }
             }
           }
-        }
-        __syncwarp();  // lane 0's acquire covers the loads of all lanes (a vote orders no memory)
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        float mx = -INFINITY, l = 0.f;
-        if (i < p.M) {
-          const float2* st = chunk_state + (size_t)g.bh * p.m_pad + i;
-          const size_t step = (size_t)p.BH * p.m_pad;
-          constexpr int kBatch = 16;  // loads in flight
-          for (int s0 = 0; s0 < S; s0 += kBatch) {
-            float2 v[kBatch];
-            float top = mx;
+          __syncwarp();  // lane 0's acquire covers the loads of all lanes (a vote orders no memory)
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          float mx = -INFINITY, l = 0.f;
+          if (i < p.M) {
+            const float2* st = chunk_state + (size_t)g.bh * p.m_pad + i;
+            const size_t step = (size_t)p.BH * p.m_pad;
+            constexpr int kBatch = 16;  // loads in flight
+            for (int s0 = 0; s0 < S; s0 += kBatch) {
+              float2 v[kBatch];
+              float top = mx;
 #pragma unroll
-            for (int u = 0; u < kBatch; ++u)
-              v[u] = s0 + u < S ? __ldcg(st + (size_t)(s0 + u) * step) : make_float2(-INFINITY, 0.f);
+              for (int u = 0; u < kBatch; ++u)
+                v[u] = s0 + u < S ? __ldcg(st + (size_t)(s0 + u) * step) : make_float2(-INFINITY, 0.f);
 #pragma unroll
-            for (int u = 0; u < kBatch; ++u) top = fmaxf(top, v[u].x);
-            if (mx != -INFINITY) l *= exp2f(mx - top);
-            mx = top;
+              for (int u = 0; u < kBatch; ++u) top = fmaxf(top, v[u].x);
+              if (mx != -INFINITY) l *= exp2f(mx - top);
+              mx = top;
 #pragma unroll
-            for (int u = 0; u < kBatch; ++u)  // a chunk this query does not see left (-inf, 0)
-              if (v[u].x != -INFINITY || v[u].y != 0.f) l = fmaf(v[u].y, exp2f(v[u].x - mx), l);
+              for (int u = 0; u < kBatch; ++u)  // a chunk this query does not see left (-inf, 0)
+                if (v[u].x != -INFINITY || v[u].y != 0.f) l = fmaf(v[u].y, exp2f(v[u].x - mx), l);
+            }
           }
+          lse_head = g.bh;
+          neg_lse = i < p.M ? -(mx + log2f(l)) : 0.f;
         }
         const uint32_t lb = (n_cols - 1) % kOsLseBuffers, lph = ((n_cols - 1) / kOsLseBuffers) & 1u;
         ok = WAIT_BEHIND_PEERS(bar_lse_empty(lb), lph ^ 1u, ST_OS_WAIT_LSE_EMPTY);
         if (!ok) break;
-        lse_all[lb * kTile + i] = i < p.M ? -(mx + log2f(l)) : 0.f;
+        lse_all[lb * kTile + i] = neg_lse;
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(bar_lse_full(lb));
       }
-      if (segment(r, 0, g) && (int)(n_rows++ % copies) == team) {
+      if (segment(n, 0, g) && (int)(n_rows++ % copies) == team) {
         const uint32_t pb = (n_rows - 1) % kOsPartBuffers, pph = ((n_rows - 1) / kOsPartBuffers) & 1u;
         ok = WAIT_BEHIND_PEERS(bar_part_full(pb), pph, ST_OS_WAIT_PART_FULL);
         if (!ok) break;
@@ -422,6 +434,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (lane == 0) ptx::red_release_add(head_count + (size_t)g.bh * kOsStatWarps + w, 1);
         __syncwarp();
       }
+      record_done(n);
     }
   } else {
     // -------------------------------------------------------- softmax warps
@@ -436,12 +449,11 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const bool live = first_q < p.M;
     uint32_t seq = 0, n_rows = 0, n_cols = 0;  // tiles and segments so far
     bool ok = true;
-    Record r;
-    for (uint32_t n = 0; ok && next_record(n, r, ok); ++n) {
+    for (uint32_t n = 0; ok && next_record(n, ok); ++n) {
 #pragma unroll 1  // (unrolled, the sum reduction spills two of its 80 registers)
       for (int kind = 0; kind < 2; ++kind) {
         Segment g;
-        if (!ok || !segment(r, kind, g)) continue;
+        if (!ok || !segment(n, kind, g)) continue;
         const int j0 = (int)((uint32_t)(wg - (int)seq) & (kKsBuffers - 1));  // my first tile within the chunk
         const uint32_t seq0 = seq;
         seq += (uint32_t)(g.t_hi - g.t_lo);
@@ -538,6 +550,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           if (lane == 0) ptx::mbar_arrive(bar_lse_empty(lb));  // done with these lse values
         }
       }
+      if (ok) record_done(n);
     }
   }
 

@@ -80,7 +80,7 @@ class _Cta:
         self.parts_full, self.parts_read = 0, set()
         self.lse_full, self.lse_done = set(), 0
         self.agents = [self.tma(), self.fold()] + [self.stat(t) for t in range(sim.copies)]
-        self.read = {x: 0 for x in range(1 + sim.copies)}  # records read: by the folding warps, by each team
+        self.read = {x: -1 for x in range(1 + sim.copies)}  # the record at hand: of the folding warps, of each team
 
     def segment(self, item, kind):
         _, _, lo, hi = self.sim.item(self.sim.S, self.sim.tiles, item)
@@ -105,24 +105,23 @@ class _Cta:
             self.records.append(rec)
             return rec
 
-        rec, first = announce(), True
+        rec = announce()
         while rec is not None:
             need = sim.lib.dealer_needs_ticket(d)
-            ticket = sim.draw() if need and not first else None
             if rec[0] >= 0:
                 yield from self.segment(rec[0], 0)
             if need:
-                sim.lib.dealer_draw(d, sim.draw() if first else ticket)
-            yield lambda: len(self.records) - min(self.read.values()) < 16
-            cols, rec, first = rec[1], announce(), False
+                sim.lib.dealer_draw(d, sim.draw())
+            yield lambda: len(self.records) - max(0, min(self.read.values())) < 16
+            cols, rec = rec[1], announce()
             if cols >= 0:
                 yield from self.segment(cols, 1)
         sim.lib.dealer_free(d)
 
     def next_record(self, reader):
+        self.read[reader] += 1  # the one before is given back
         yield lambda: len(self.records) > self.read[reader]
-        self.read[reader] += 1
-        return self.records[self.read[reader] - 1]
+        return self.records[self.read[reader]]
 
     def fold(self):
         n_rows = n_cols = 0
