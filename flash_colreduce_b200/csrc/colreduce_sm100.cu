@@ -537,7 +537,8 @@ pass_kernel(const __grid_constant__ CUtensorMap tmap_stat,
               // its issuer is the instructions around the MMAs, not the MMAs: with two 64-bit descriptors put
               // together per step and a lane test that made every operand divergent, a tile of eight took 850
               // cycles to issue (its MMAs take 512); with the descriptors' lower halves stepped by a constant
-              // under an elected lane 610.  8 heads of 131072^2: 38.7 -> 38.1 ms; 512 heads of 1024^2: 380 -> 371 us.
+              // under an elected lane 610.  (8 heads of 131072^2 38.7 -> 38.1 ms, 512 heads of 1024^2 380 -> 371 us: about
+              // what the runs of one build differ by.  At the power cap saved cycles come back as a lower clock.)
               // The operand kind is chosen once, outside the unrolled sequence.
               constexpr int kSteps = DPAD / 16 / L::kPieces;  // instructions per ring slot
               const uint32_t a_lo = ptx::smem_desc_lo(a_addr) + piece * (L::kSlotHalves * (L::kHalfBytes >> 4));

@@ -15,11 +15,13 @@
 // are free.  Dealt round-robin to CTAs that all had to be resident (a cooperative launch), it could not even start
 // while a kernel of another stream held one SM.
 //
-// Measured (whole call, sustained): 16 x 32 heads, 64 x 16384, d = 128, fp16: 876 us in two sweeps, 640 in one;
-// 8 heads, 64 x 32768: 43 -> 27; one head, 64 x 60000: 85 -> 21 (few heads: the combination of many partial
-// states and two launches go too); 32 heads, 128 x 4096: 26 -> 24.  What bounds the large one now is power: the
-// board sits at its 1000 W cap with the SMs at 1.4 GHz (in a burst of a few calls it takes 563 us against 696);
-// DRAM reads equal K's size (541 MB for 537 MB), MUFU 27 %, tensor pipe 21 %.
+// Measured (us per call in a graph, sustained, fp16, on one board): 16 x 32 heads, 64 x 16384, d = 128: 888 in two
+// sweeps, 680 here; 8 heads, 64 x 32768: 46.6 -> 26.7; one head, 64 x 60000: 81 -> 20.5 (few heads: the combination of
+// many partial states and two launches go too); 32 heads, 128 x 4096: 26.8 -> 23.3; 2 heads, 128 x 100000: 83 -> 43.
+// (Dealt round-robin under a cooperative launch the same five took 674, 24.7, 20.4, 22.6 and 39: the tickets cost up to
+// a tenth where a CTA has two long chunks, and nothing to speak of elsewhere.)  What bounds the large one is power: the
+// board sits at its 1000 W cap with the SMs at 1.4 GHz.  On a quarter of that batch DRAM reads are 563 MB for 537 MB of
+// K, MUFU is busy for 39 %, the tensor pipe for 37 %, the issue slots for 47 % of the time.
 //
 // Spare rows of the 128-row MMA repeat the query tile (2 copies for M <= 64, 4 for M <= 32), so that in the rows
 // pass the warps of those lanes fold their own share of a key tile's columns; with one copy two of the four
@@ -33,7 +35,7 @@
 
 namespace fcr {
 
-constexpr int kOsMmaWarps = 2;  // take the tiles in turn: issuing one costs a warp about 1000 cycles with its waits, its MMAs take 256 to 512 (one warp: 812 us where two took 770)
+constexpr int kOsMmaWarps = 2;  // take the tiles in turn: issuing one costs a warp about 1000 cycles with its waits, its MMAs take 256 to 512 (16 x 32 heads, 64 x 16384: 728 us with one warp, 671 with two)
 constexpr int kOsStatWarp = kKsMmaWarp + kOsMmaWarps;
 constexpr int kOsStatWarps = 4;
 constexpr int kOsThreads = (kOsStatWarp + kOsStatWarps) * 32;
@@ -199,7 +201,7 @@ onesweep_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   if (warp == kKsProducerWarp) {
     // ------------------------------------------------------------ TMA warp
     // A rows segment's tiles are wanted once more, a columns segment's never again: told so, the L2 gives up the
-    // latter first (without the hint the large batch above takes 812 us, its second sweep missing half the time).
+    // latter first (the large batch above took 795 to 808 us without the hint where it took 671 with it).
     const uint64_t keep = ptx::l2_policy_evict_normal(), drop = ptx::l2_policy_evict_first();
     uint32_t ring_seq = 0, q_seq[2] = {0, 0};
     bool ok = true;

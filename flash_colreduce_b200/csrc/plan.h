@@ -201,12 +201,13 @@ inline int choose_splits(int64_t base_items, int64_t max_len_tiles, int num_sms)
 
 // One-sweep decode kernel (onesweep_sm100.cuh): chunks per head, 0 when the plan does not take it.
 // It takes the key-streaming shapes without a score cache whose operand rows span at most 256 bytes (two
-// query tiles of 64 KB would leave no room for a key ring).  CTA c runs chunks c, c + G, ... and reads a
-// chunk's tiles again one chunk later.  Unless all of K fits the L2 anyway, a chunk is at most 256 KB of K:
+// query tiles of 64 KB would leave no room for a key ring).  A CTA reads a
+// chunk's tiles again one chunk later (OneSweepDealer).  Unless all of K fits the L2 anyway, a chunk is at most 256 KB of K:
 // 16 x 32 heads, 64 x 16384, d = 128 took 1046 us with chunks of 3 tiles of 32 KB, 767 with 5, 665 with 8 and
-// 696 with 10 (two sweeps: 876), the small ones for the set-up of a chunk (about two tiles' time, the 2 in the
+// 696 with 10 (two sweeps: 876; measured on the kernel's first, cooperative form), the small ones for the set-up of a chunk (about two tiles' time, the 2 in the
 // cost below), the large ones because the chunk has left the L2 before its second sweep.  S <= num_sms, so that on
 // an idle GPU a CTA's next ticket lies beyond the head of its last one and each chunk is reduced one ticket later.
+// (Bytes are those of padded rows: d = 80 and 96 get the chunks and the L2 test of d = 128.)
 // With rows of 128 bytes and more than 64 queries the folds bind, not the reading of K, and the second sweep
 // saves nothing: 256 heads, 128 x 8192, d = 64 took 158 us in two sweeps, 167 in one.  Only where K fits the
 // L2, whose problems are bound by the launches and the combination instead (4 heads, 128 x 65536: 56 -> 32 us).

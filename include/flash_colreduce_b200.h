@@ -114,9 +114,12 @@ typedef struct fcr_plan {
   /* Key streaming without a score cache and with operand rows of at most 256 bytes: one kernel runs both
    * passes chunk by chunk, so that K is read from HBM once, when the workspace has workspace_bytes bytes.
    * Its scratch (chunk counters and chunk states) is the last region of the workspace and optional: a
-   * workspace that ends after off_part_l's array is accepted, and the two kernels described above run. */
+   * workspace that ends after off_part_l's array is accepted, and the two kernels described above run.
+   * The fields of this struct (key_chunks, row_splits, the items and CTAs) and fcr_plan_item describe those two
+   * kernels for such a problem too; the one-sweep kernel's chunks follow from the problem and the SM count. */
   int32_t static_schedule;  /* 1: work items are dealt round-robin (item, item + CTAs, ...) and nothing in the workspace has
-                             * to be cleared before the kernels (small problems and the key-streaming kernels);
+                             * to be cleared before the kernels (small problems and the key-streaming kernels; the
+                             * one-sweep kernel's counters are cleared by a cudaMemsetAsync of their own);
                              * 0: CTAs draw items from a counter, which one cudaMemsetAsync per call clears */
 } fcr_plan;
 
