@@ -208,16 +208,16 @@ inline int choose_splits(int64_t base_items, int64_t max_len_tiles, int num_sms)
 // cost below), the large ones because the chunk has left the L2 before its second sweep.  S <= num_sms, so that on
 // an idle GPU a CTA's next ticket lies beyond the head of its last one and each chunk is reduced one ticket later.
 // (Bytes are those of padded rows: d = 80 and 96 get the chunks and the L2 test of d = 128.)
-// With rows of 128 bytes and more than 64 queries the folds bind, not the reading of K, and the second sweep
-// saves nothing: 256 heads, 128 x 8192, d = 64 took 158 us in two sweeps, 167 in one.  Only where K fits the
-// L2, whose problems are bound by the launches and the combination instead (4 heads, 128 x 65536: 56 -> 32 us).
+// With rows of 128 bytes and more than 64 queries the folds weigh as much as the reading of K, and one sweep still
+// gains: 256 heads, 8192 keys, d = 64 took 181 us with 128 queries in two sweeps and 162 in one, 163 and 144 with 96,
+// 174 and 153 with 72 (sustained); where K fits the L2 the launches and the combination go too (4 heads, 128 x 65536:
+// 57 -> 31 us).
 constexpr int64_t kOneSweepL2Bytes = 40LL << 20;
 constexpr int64_t kOneSweepChunkBytes = 256 << 10;
 inline int onesweep_chunks(const fcr_problem& p, const fcr_plan& pl, int num_sms) {
   if (!pl.key_stream || pl.score_cache || pl.d_pad > 128) return 0;
   const int64_t BH = (int64_t)p.B * p.H, key_tiles = pl.n_pad / kTile, tile_bytes = (int64_t)kTile * pl.d_pad * 2;
   const bool in_l2 = BH * key_tiles * tile_bytes <= kOneSweepL2Bytes;
-  if (!in_l2 && pl.d_pad == 64 && p.M > 64) return 0;
   int best = 0;
   int64_t best_cost = -1;
   for (int64_t s = 1; s <= std::min<int64_t>(key_tiles, std::min(num_sms, kOneSweepHeld)); ++s) {

@@ -247,7 +247,7 @@ def test_the_chunks_are_chosen_with_the_plan():
 
 def test_which_shapes_take_it_and_where_its_scratch_lies(planner):
     plan, _, _ = planner
-    for m, n, d, dtype, takes in [(17, 1024, 128, 0, True), (128, 1024, 64, 0, True), (64, 4096, 80, 1, True), (64, 4096, 64, 2, True),
+    for m, n, d, dtype, takes in [(17, 1024, 128, 0, True), (100, 90000, 64, 0, True), (128, 1024, 64, 0, True), (64, 4096, 80, 1, True), (64, 4096, 64, 2, True),
                                   (16, 4096, 128, 0, False),   # score cache
                                   (64, 4096, 129, 0, False), (64, 4096, 72, 2, False),  # rows beyond 256 bytes
                                   (64, 800000, 128, 0, False),  # too few, too long heads: a chunk would outgrow the L2
@@ -286,6 +286,7 @@ def _call(nat, qd, kd, red, causal, scale, ws_bytes=None):
                                              (3, 50, 64, 1151, 128, "fp16"),  # several heads per CTA
                                              (2, 75, 32, 6000, 64, "bf16"),   # four teams, ten chunks per CTA
                                              (1, 2, 100, 20000, 64, "fp32"),  # TF32, long head
+                                             (4, 80, 100, 2100, 64, "bf16"),  # short rows, K beyond the L2
                                              (1, 160, 128, 1300, 128, "bf16"),
                                              (1, 1, 127, 70001, 128, "fp16")])  # one head over all CTAs, several chunks each
 def test_one_sweep_matches_the_oracle_and_the_two_sweep_kernels(b, h, m, n, d, dtype):
